@@ -391,14 +391,10 @@ Batch::Batch(int nrep, const tdmd_box* boxes, const int* natoms, const tdmd_mors
     row_filter_band(d.box, rl2_, &d.lo_f, &d.hi_f, &d.wrap);
     RepScale& s = sc[static_cast<size_t>(r)];
     s = RepScale{};
-    RepImg& m = img[static_cast<size_t>(r)];
-    m = RepImg{};
+    img[static_cast<size_t>(r)] = img3(d.box);
     for (int a = 0; a < 3; ++a) {
       s.s[a] = d.box.qscale[a];
       s.s2[a] = d.box.qstep[a] * d.box.qstep[a];
-      m.L[a] = d.box.L[a];
-      m.halfL[a] = d.box.halfL[a];
-      m.per[a] = d.box.periodic[a];
     }
     s.iso = d.box.qstep[0] == d.box.qstep[1] && d.box.qstep[1] == d.box.qstep[2];
     atoms += natoms[r];

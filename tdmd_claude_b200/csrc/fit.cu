@@ -56,10 +56,7 @@ struct SplC {
 };
 
 __device__ __forceinline__ int spl_seg(double x, double step, int ns, double& dx) {
-  int k = static_cast<int>(x / step);
-  k = k < 0 ? 0 : (k >= ns ? ns - 1 : k);
-  dx = x - static_cast<double>(k) * step;
-  return k;
+  return spline_idx(x, step, ns + 1, dx);
 }
 
 template <class T>
@@ -76,6 +73,12 @@ __device__ __forceinline__ T spl_deriv(const SplC& s, int k, T dx) {
   const T c = static_cast<T>(__ldg(s.c + 2 * s.ns + k)),
           d = static_cast<T>(__ldg(s.c + 3 * s.ns + k));
   return b + dx * (T(2) * c + T(3) * d * dx);
+}
+
+// 1/r as a double: the FP64 geometries' own, a division of the FP32 radius.
+__device__ __forceinline__ double inv_radius(double /*r*/, double rinv) { return rinv; }
+__device__ __forceinline__ double inv_radius(float r, float /*rinv*/) {
+  return 1.0 / static_cast<double>(r);
 }
 
 // Gradient scatter into a packed a|b|c|d spline gradient.
@@ -110,7 +113,7 @@ struct FitEam {
   double* grho;
   double* gphi;
   int nt, nsf, nsr;
-  double drho, dr;
+  double drho, dr, inv_dr;
   __device__ __forceinline__ SplC Fs(int t) const { return SplC{F + 4ll * nsf * t, nsf, drho}; }
   __device__ __forceinline__ SplC rhos(int t) const {
     return SplC{rho + 4ll * nsr * t, nsr, dr};
@@ -166,7 +169,7 @@ __global__ void __launch_bounds__(kThreads) k_fm_morse_force(
         double rd;
         g.radius(o, pr, r, rinv, rd);
         const T ex = exp(-alpha * static_cast<T>(rd - r0d));
-        const T fpair = -over_r(T(2) * D * alpha * (T(1) - ex) * ex, r, rinv);
+        const T fpair = -div_r(T(2) * D * alpha * (T(1) - ex) * ex, r, rinv);
         fx.add(mul_rn(fpair, pr.dx));
         fy.add(mul_rn(fpair, pr.dy));
         fz.add(mul_rn(fpair, pr.dz));
@@ -220,7 +223,7 @@ __global__ void __launch_bounds__(kThreads) k_fm_morse_grad(Geo g, NbrView nl, i
         const T ex = exp(-at * static_cast<T>(rd - r0));
         const T ome = T(1) - ex;
         const double gd = (gx * static_cast<double>(pr.dx) + gy * static_cast<double>(pr.dy) +
-                           gz * static_cast<double>(pr.dz)) / static_cast<double>(r);
+                           gz * static_cast<double>(pr.dz)) * inv_radius(r, rinv);
         // df/dtheta * r (the 1/r is folded into gd)
         const T dD = -T(2) * at * ome * ex;
         const T da = -T(2) * Dt * (ome * ex - at * (T(1) - T(2) * ex) *
@@ -275,7 +278,7 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_density(
         double rd;
         g.radius(o, pr, r, rinv, rd);
         double dx;
-        const int kk = spl_seg(rd, e.dr, e.nsr, dx);
+        const int kk = spline_idx_mul(rd, e.dr, e.inv_dr, e.nsr + 1, dx);
         rho.add(spl_value<T>(e.rhos(__ldg(types + j) - 1), kk, static_cast<T>(dx)));
       }
     }
@@ -320,12 +323,12 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_force(
         g.radius(o, pr, r, rinv, rd);
         const int tj = __ldg(types + j) - 1;
         double dxd;
-        const int kk = spl_seg(rd, e.dr, e.nsr, dxd);
+        const int kk = spline_idx_mul(rd, e.dr, e.inv_dr, e.nsr + 1, dxd);
         const T dx = static_cast<T>(dxd);
         const T dphi = spl_deriv<T>(e.phis(pair_index(ti, tj, e.nt)), kk, dx);
         const T drj = spl_deriv<T>(e.rhos(tj), kk, dx);
         const T dri = ti == tj ? drj : spl_deriv<T>(e.rhos(ti), kk, dx);
-        const T fpair = -over_r(dphi + fpi * drj + static_cast<T>(fp[j]) * dri, r, rinv);
+        const T fpair = -div_r(dphi + fpi * drj + static_cast<T>(fp[j]) * dri, r, rinv);
         fx.add(mul_rn(fpair, pr.dx));
         fy.add(mul_rn(fpair, pr.dy));
         fz.add(mul_rn(fpair, pr.dz));
@@ -382,9 +385,9 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_adjoint(
         g.radius(o, pr, r, rinv, rd);
         const int tj = __ldg(types + j) - 1;
         double dx;
-        const int kk = spl_seg(rd, e.dr, e.nsr, dx);
-        const double ddx = pr.dx, ddy = pr.dy, ddz = pr.dz, rr = static_cast<double>(r);
-        const double q = (gix * ddx + giy * ddy + giz * ddz) / rr;
+        const int kk = spline_idx_mul(rd, e.dr, e.inv_dr, e.nsr + 1, dx);
+        const double ddx = pr.dx, ddy = pr.dy, ddz = pr.dz, ri = inv_radius(r, rinv);
+        const double q = (gix * ddx + giy * ddy + giz * ddz) * ri;
         const double fpj = fp[j];
         add_deriv_basis(e.gphi + 4ll * e.nsr * pair_index(ti, tj, e.nt), e.nsr, kk, dx, -q);
         if (ti == tj) {
@@ -396,7 +399,7 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_adjoint(
         const double drj = spl_deriv<double>(e.rhos(tj), kk, dx);
         const double gdiff = (gix - G[3ll * j]) * ddx + (giy - G[3ll * j + 1]) * ddy +
                              (giz - G[3ll * j + 2]) * ddz;
-        w -= drj * gdiff / rr;
+        w -= drj * gdiff * ri;
       }
     }
   }
@@ -419,7 +422,7 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_adjoint(
       g.radius(o, pr, r, rinv, rd);
       const int tj = __ldg(types + j) - 1;
       double dx;
-      const int kk = spl_seg(rd, e.dr, e.nsr, dx);
+      const int kk = spline_idx_mul(rd, e.dr, e.inv_dr, e.nsr + 1, dx);
       add_value_basis(e.grho + 4ll * e.nsr * tj, e.nsr, kk, dx, wf);
     }
   }
@@ -475,9 +478,9 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_adjoint_w(
           double rd;
           g.radius(o, pr, r, rinv, rd);
           double dx;
-          const int kk = spl_seg(rd, e.dr, ns, dx);
-          const double ddx = pr.dx, ddy = pr.dy, ddz = pr.dz, rr = static_cast<double>(r);
-          const double q = (gix * ddx + giy * ddy + giz * ddz) / rr;
+          const int kk = spline_idx_mul(rd, e.dr, e.inv_dr, ns + 1, dx);
+          const double ddx = pr.dx, ddy = pr.dy, ddz = pr.dz, ri = inv_radius(r, rinv);
+          const double q = (gix * ddx + giy * ddy + giz * ddz) * ri;
           const double fpj = fp[j];
           // phi' and rho' terms: d/dc of the derivative basis (b, 2c x, 3d x^2)
           const double wp = -q, wr = -q * (fpi + fpj);
@@ -490,7 +493,7 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_adjoint_w(
           const double drj = spl_deriv<double>(e.rhos(0), kk, dx);
           const double gdiff = (gix - G[3ll * j]) * ddx + (giy - G[3ll * j + 1]) * ddy +
                                (giz - G[3ll * j + 2]) * ddz;
-          w -= drj * gdiff / rr;
+          w -= drj * gdiff * ri;
         }
       }
     }
@@ -512,7 +515,7 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_adjoint_w(
           double rd;
           g.radius(o, pr, r, rinv, rd);
           double dx;
-          const int kk = spl_seg(rd, e.dr, ns, dx);
+          const int kk = spline_idx_mul(rd, e.dr, e.inv_dr, ns + 1, dx);
           add_r(e.grho, srho, ns, kk, k0, W, 0, wf);
           add_r(e.grho, srho, ns, kk, k0, W, 1, wf * dx);
           add_r(e.grho, srho, ns, kk, k0, W, 2, wf * dx * dx);
@@ -625,7 +628,7 @@ Fit::Fit(int nsnap, int natoms, const tdmd_box& box, const double* pos, const in
     p4[i] = make_double4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], static_cast<double>(types[i]));
   }
   const RepScale sc = rep_scale(b);
-  const RepImg im = rep_img(b);
+  const RepImg im = img3(b);
   std::vector<RepScale> scv(static_cast<size_t>(nsnap), sc);
   std::vector<RepImg> imv(static_cast<size_t>(nsnap), im);
   cudaStream_t s = nullptr;
@@ -755,7 +758,7 @@ void Fit::eam(int ntypes, int nrho, double drho, int nr, double dr, const double
   const bool grad = gF || grho || gphi;
   TDMD_REQUIRE(!grad || (gF && grho && gphi), "give all three gradient arrays or none");
   const int npairs = ntypes * (ntypes + 1) / 2;
-  FitEam e{F, rho, phi, gF, grho, gphi, ntypes, nrho - 1, nr - 1, drho, dr};
+  FitEam e{F, rho, phi, gF, grho, gphi, ntypes, nrho - 1, nr - 1, drho, dr, 1.0 / dr};
   if (grad) {
     TDMD_CU(cudaMemsetAsync(gF, 0, sizeof(double) * 4 * (nrho - 1) * ntypes, s));
     TDMD_CU(cudaMemsetAsync(grho, 0, sizeof(double) * 4 * (nr - 1) * ntypes, s));

@@ -456,8 +456,7 @@ int32_t tdmd_morse_compute(const double* d_positions, void* d_forces, int32_t pr
     const int nblk = force_blocks(natoms, lpa);
     Partials part(ev ? nblk : 0, s);
     if (precision == TDMD_FP64) {
-      GeoAoS64 g{d_positions, {b.L[0], b.L[1], b.L[2]}, {b.halfL[0], b.halfL[1], b.halfL[2]},
-                 {b.periodic[0], b.periodic[1], b.periodic[2]}};
+      const GeoAoS64 g{d_positions, img3(b)};
       MorseP<double> mp{params->d, params->alpha, params->r0, params->rc_sq, params->r0};
       launch_morse(g, nl, natoms, mp, static_cast<double*>(d_forces), ev, part.p, lpa, s);
     } else {
@@ -493,8 +492,7 @@ int32_t tdmd_morse_compute_zone(const double* d_positions, void* d_forces, int32
     const int nblk = force_blocks(atom_count, lpa);
     Partials part(ev ? nblk : 0, s);
     if (precision == TDMD_FP64) {
-      GeoAoS64 g{d_positions, {b.L[0], b.L[1], b.L[2]}, {b.halfL[0], b.halfL[1], b.halfL[2]},
-                 {b.periodic[0], b.periodic[1], b.periodic[2]}};
+      const GeoAoS64 g{d_positions, img3(b)};
       MorseP<double> mp{params->d, params->alpha, params->r0, params->rc_sq, params->r0};
       launch_morse_zone(g, first_atom, nl, atom_count, mp, static_cast<double*>(d_forces), ev,
                         part.p, lpa, s);
@@ -561,8 +559,7 @@ int32_t tdmd_device_eam_compute(tdmd_device_eam* de, const double* d_positions, 
     const int* types = de->tabs.ntypes > 1 ? d_types : nullptr;
     if (precision == TDMD_FP64) {
       de->fp64.reserve(static_cast<size_t>(natoms));
-      GeoAoS64 g{d_positions, {b.L[0], b.L[1], b.L[2]}, {b.halfL[0], b.halfL[1], b.halfL[2]},
-                 {b.periodic[0], b.periodic[1], b.periodic[2]}};
+      const GeoAoS64 g{d_positions, img3(b)};
       launch_eam(g, nl, natoms, de->tabs.d64, types, de->fp64.data(), d_rho, d_fp,
                  static_cast<double*>(d_forces), ev, part.p, lpa, s);
     } else {

@@ -101,8 +101,7 @@ extern "C" int32_t tdmd_morse_compute_noalloc(const double* d_positions, void* d
     TDMD_REQUIRE(nblk <= kMaxBlocks, "partial records exceed the fixed scratch");
     double* part = ev ? scratch_for_current_device() : nullptr;
     if (precision == TDMD_FP64) {
-      GeoAoS64 g{d_positions, {b.L[0], b.L[1], b.L[2]}, {b.halfL[0], b.halfL[1], b.halfL[2]},
-                 {b.periodic[0], b.periodic[1], b.periodic[2]}};
+      const GeoAoS64 g{d_positions, img3(b)};
       MorseP<double> mp{params->d, params->alpha, params->r0, params->rc_sq, params->r0};
       launch_morse(g, nl, natoms, mp, static_cast<double*>(d_forces), ev, part, lpa, s);
     } else {

@@ -10,11 +10,7 @@
 namespace tdmd_b200 {
 
 // Per-replica minimum-image constants of the FP64 path.
-struct RepImg {
-  double L[3], halfL[3];
-  int per[3];
-  int pad;
-};
+using RepImg = Img3;
 
 // Mixed: fixed-point records, per-replica decode scales (the center atom's
 // replica; all of its neighbors share it).
@@ -73,7 +69,6 @@ struct GeoD4B {
   struct Own {
     double x, y, z;
     double L0, L1, L2, h0, h1, h2;
-    int p0, p1, p2;
   };
   using Pair = PairD;
   static constexpr bool kRecords = false;
@@ -94,28 +89,28 @@ struct GeoD4B {
     o.L0 = __ldg(&m->L[0]);
     o.L1 = __ldg(&m->L[1]);
     o.L2 = __ldg(&m->L[2]);
-    o.h0 = __ldg(&m->halfL[0]);
-    o.h1 = __ldg(&m->halfL[1]);
-    o.h2 = __ldg(&m->halfL[2]);
-    o.p0 = __ldg(&m->per[0]);
-    o.p1 = __ldg(&m->per[1]);
-    o.p2 = __ldg(&m->per[2]);
+    o.h0 = __ldg(&m->h[0]);
+    o.h1 = __ldg(&m->h[1]);
+    o.h2 = __ldg(&m->h[2]);
     return o;
   }
   __device__ __forceinline__ void pair(const Own& o, int j, Pair& pr) const {
     const double3 q = load(j);
-    pr.dx = min_image1(o.x - q.x, o.L0, o.h0, o.p0);
-    pr.dy = min_image1(o.y - q.y, o.L1, o.h1, o.p1);
-    pr.dz = min_image1(o.z - q.z, o.L2, o.h2, o.p2);
+    pr.dx = image1(o.x - q.x, o.L0, o.h0);
+    pr.dy = image1(o.y - q.y, o.L1, o.h1);
+    pr.dz = image1(o.z - q.z, o.L2, o.h2);
     pr.r2 = pr.dx * pr.dx + pr.dy * pr.dy + pr.dz * pr.dz;
   }
   __device__ __forceinline__ void radius(const Own&, const Pair& pr, T& r, T& rinv,
                                          double& rd) const {
-    r = sqrt(pr.r2);
-    rinv = 1.0 / r;
+    radius_d(pr.r2, r, rinv);
     rd = r;
   }
-  __device__ __forceinline__ T radius_fast(const Pair& pr) const { return sqrt(pr.r2); }
+  __device__ __forceinline__ T radius_fast(const Pair& pr) const {
+    T r, rinv;
+    radius_d(pr.r2, r, rinv);
+    return r;
+  }
 };
 
 // FP64 gather records {x, y, z, F'(rho)} of a batch (written by the
@@ -134,33 +129,26 @@ struct GeoD4BF {
   }
   __device__ __forceinline__ void pair(const Own& o, int j, Pair& pr) const {
     const double4 q = ld_d4(p + j);
-    pr.dx = min_image1(o.x - q.x, o.L0, o.h0, o.p0);
-    pr.dy = min_image1(o.y - q.y, o.L1, o.h1, o.p1);
-    pr.dz = min_image1(o.z - q.z, o.L2, o.h2, o.p2);
+    pr.dx = image1(o.x - q.x, o.L0, o.h0);
+    pr.dy = image1(o.y - q.y, o.L1, o.h1);
+    pr.dz = image1(o.z - q.z, o.L2, o.h2);
     pr.r2 = pr.dx * pr.dx + pr.dy * pr.dy + pr.dz * pr.dz;
     pr.fw = q.w;
   }
   __device__ __forceinline__ void radius(const Own&, const Pair& pr, T& r, T& rinv,
                                          double& rd) const {
-    r = sqrt(pr.r2);
-    rinv = 1.0 / r;
+    radius_d(pr.r2, r, rinv);
     rd = r;
   }
-  __device__ __forceinline__ T radius_fast(const Pair& pr) const { return sqrt(pr.r2); }
+  __device__ __forceinline__ T radius_fast(const Pair& pr) const {
+    T r, rinv;
+    radius_d(pr.r2, r, rinv);
+    return r;
+  }
   __device__ __forceinline__ double gather_fp(const Pair& pr, int /*tmask*/) const {
     return pr.fw;
   }
 };
-
-__host__ inline RepImg rep_img(const DevBox& b) {
-  RepImg m{};
-  for (int a = 0; a < 3; ++a) {
-    m.L[a] = b.L[a];
-    m.halfL[a] = b.halfL[a];
-    m.per[a] = b.periodic[a];
-  }
-  return m;
-}
 
 __host__ inline RepScale rep_scale(const DevBox& b) {
   RepScale s{};

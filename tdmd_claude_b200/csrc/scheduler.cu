@@ -802,9 +802,7 @@ void Scheduler::enqueue_force(bool ev, bool kd, int parts) {
       const GeoQ g = make_geoq(q_.data(), box_);
       launch_morse(g, nl, n_, m32_, f32_.data(), ev, part, tf, s);
     } else {
-      GeoD4 g{pos4_.data(), {box_.L[0], box_.L[1], box_.L[2]},
-              {box_.halfL[0], box_.halfL[1], box_.halfL[2]},
-              {box_.periodic[0], box_.periodic[1], box_.periodic[2]}};
+      const GeoD4 g{pos4_.data(), img3(box_)};
       launch_morse(g, nl, n_, m64_, f64_.data(), ev, part, tf, s);
     }
     prof_end(kProfForce);
@@ -838,12 +836,8 @@ void Scheduler::enqueue_force(bool ev, bool kd, int parts) {
     } else {
       // Density reads the position records and writes {x, y, z, F'} gather
       // records; the force pass gathers those.
-      GeoD4 g{pos4_.data(), {box_.L[0], box_.L[1], box_.L[2]},
-              {box_.halfL[0], box_.halfL[1], box_.halfL[2]},
-              {box_.periodic[0], box_.periodic[1], box_.periodic[2]}};
-      GeoD4F gg{g64_.data(), {box_.L[0], box_.L[1], box_.L[2]},
-                {box_.halfL[0], box_.halfL[1], box_.halfL[2]},
-                {box_.periodic[0], box_.periodic[1], box_.periodic[2]}};
+      const GeoD4 g{pos4_.data(), img3(box_)};
+      const GeoD4F gg{g64_.data(), img3(box_)};
       if (parts & kPassDensity) {
         prof_begin(kProfDensity);
         launch_eam_density<GeoD4, double>(g, nl, n_, eam_->d64, types, fp64_.data(), nullptr,

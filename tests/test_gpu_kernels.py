@@ -1,0 +1,66 @@
+"""Edges of the kernels' ranges: branches of the pair arithmetic, of the list
+build and of the force-matching adjoint, at the sizes where they change."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(torch, a, dtype=None):
+    return torch.as_tensor(np.ascontiguousarray(a), device="cuda", dtype=dtype)
+
+
+def _spline(c, x, h):
+    """(value, derivative) of packed a|b|c|d coefficients at x."""
+    ns = len(c) // 4
+    k = min(max(int(x / h), 0), ns - 1)
+    dx = x - k * h
+    a, b, cc, d = (c[m * ns + k] for m in range(4))
+    return a + dx * (b + dx * (cc + dx * d)), b + dx * (2 * cc + 3 * d * dx)
+
+
+# below the FP32 seed's range, tiny, on spline knots (dr = 5/1999), ordinary, at
+# the cutoff's two sides
+@pytest.mark.parametrize("r", [1e-18, 1e-3, 400 * 5 / 1999, 1000 * 5 / 1999, 2.556, 4.9999999, 5.0])
+@pytest.mark.parametrize("wrapped", [False, True])
+def test_fp64_pair_radius(cuda, r, wrapped):
+    """Two atoms r apart, directly or through the periodic face: density, F'
+    and force against numpy's square root and divisions.  A rounding of r
+    moves phi' by |phi''/phi'| ulp(r) < 20 ulp: 1e-14 relative, ten times
+    that allowed."""
+    from tdmd_claude_b200 import Box, DeviceEam, EamAlloy
+    from tdmd_claude_b200 import workloads as W
+    t = W.cu_eam_tables()
+    eam = EamAlloy.from_tables(t.ntypes, t.nrho, t.drho, t.nr, t.dr, t.cutoff, t.F, t.rho, t.rphi)
+    lo, hi = -10.0, 22.0
+    pos = np.array([[lo, 1.0, 2.0], [hi - r, 1.0, 2.0]] if wrapped else
+                   [[0.0, 1.0, 2.0], [r, 1.0, 2.0]])
+    dx = pos[0, 0] - pos[1, 0] + ((hi - lo) if wrapped else 0.0)
+    r = abs(dx)
+    if r == 0.0:
+        pytest.skip("the face swallows this separation")
+    de = DeviceEam()
+    de.upload_tables(eam)
+    f64 = cuda.float64
+    f = cuda.zeros((2, 3), dtype=f64, device="cuda")
+    rho = cuda.zeros(2, dtype=f64, device="cuda")
+    fp = cuda.zeros(2, dtype=f64, device="cuda")
+    nbr = _dev(cuda, np.array([1, 0], np.int32))
+    off = _dev(cuda, np.array([0, 1], np.int32))
+    cnt = _dev(cuda, np.array([1, 1], np.int32))
+    de.compute(_dev(cuda, pos), f, _dev(cuda, np.ones(2, np.int32)), nbr.data_ptr(),
+               off.data_ptr(), cnt.data_ptr(), 2, Box.make((lo,) * 3, (hi,) * 3), d_rho=rho,
+               d_fp=fp)
+    want_rho = want_f = want_fp = 0.0
+    if r * r < t.cutoff ** 2:
+        want_rho, drho = _spline(eam.coeffs(1, 0), r, t.dr)
+    want_fp = _spline(eam.coeffs(0, 0), want_rho, t.drho)[1]
+    if r * r < t.cutoff ** 2:
+        want_f = -(_spline(eam.coeffs(2, 0), r, t.dr)[1] + 2 * want_fp * drho) / r * dx
+    assert np.allclose(rho.cpu(), want_rho, rtol=1e-13, atol=1e-16)
+    assert np.allclose(fp.cpu(), want_fp, rtol=1e-13)
+    got = f.cpu().numpy()
+    assert np.allclose(got[:, 0], [want_f, -want_f], rtol=1e-13, atol=1e-15)
+    assert not got[:, 1:].any()
