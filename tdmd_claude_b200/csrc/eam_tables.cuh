@@ -52,6 +52,8 @@ struct EamDevTables {
   DevArray<double4> dtab64;  // density rows (a, b, c, d)
   DevArray<float4> dtab32;
   DevArray<double4> ftab;
+  DevArray<double4> deriv4;  // one type, FP64: derivative rows split in two
+  DevArray<double2> deriv2;
   EamDev<double> d64{};
   EamDev<float> d32{};
   int ntypes = 0;

@@ -231,6 +231,21 @@ void EamDevTables::upload(const tdmd_eam& e, cudaStream_t stream) {
       f64[static_cast<size_t>(t) * nsf + k] =
           make_double4(c[k], c[nsf + k], c[2 * nsf + k], c[3 * nsf + k]);
   }
+  std::vector<double4> e4(nt == 1 ? static_cast<size_t>(nsr) : 0);
+  std::vector<double2> e2(e4.size());
+  for (size_t k = 0; k < e4.size(); ++k) {
+    const double4 r = r64[2 * k], p = r64[2 * k + 1];
+    e4[k] = make_double4(r.x, r.y, r.z, p.x);
+    e2[k] = make_double2(p.y, p.z);
+  }
+  deriv4.reserve(e4.size());
+  deriv2.reserve(e2.size());
+  if (nt == 1) {
+    TDMD_CU(cudaMemcpyAsync(deriv4.data(), e4.data(), e4.size() * sizeof(double4),
+                            cudaMemcpyHostToDevice, stream));
+    TDMD_CU(cudaMemcpyAsync(deriv2.data(), e2.data(), e2.size() * sizeof(double2),
+                            cudaMemcpyHostToDevice, stream));
+  }
   rtab64.reserve(r64.size());
   rtab32.reserve(r32.size());
   dtab64.reserve(d64h.size());
@@ -255,7 +270,8 @@ void EamDevTables::upload(const tdmd_eam& e, cudaStream_t stream) {
   if (nt > 1 && nt <= 16)
     while ((1 << tbits) < nt) ++tbits;
   d64 = EamDev<double>{dtab64.data(), rtab64.data(), ftab.data(), nt, S, e.nr, e.nrho, e.dr,
-                       1.0 / e.dr, e.cutoff * e.cutoff, e.drho, e.dr, 0.0, 0};
+                       1.0 / e.dr, e.cutoff * e.cutoff, e.drho, e.dr, 0.0, 0, deriv4.data(),
+                       deriv2.data()};
   const float dr32 = static_cast<float>(e.dr);
   d32 = EamDev<float>{dtab32.data(), rtab32.data(), ftab.data(), nt, S, e.nr, e.nrho, dr32,
                       static_cast<float>(1.0 / e.dr), static_cast<float>(e.cutoff * e.cutoff),

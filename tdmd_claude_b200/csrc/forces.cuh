@@ -648,6 +648,10 @@ struct EamDev {
   // F' below 2^(tbits-23)), so the force pass gathers no type; 0 = types are
   // gathered (one type, or more than 16).
   int tbits;
+  // One type, FP64, forces only: the six derivative coefficients of a bin as
+  // (rho' b, 2c, 3d, phi' b) and (phi' 2c, 3d).
+  const double4* d4 = nullptr;
+  const double2* d2 = nullptr;
 };
 
 __device__ __forceinline__ int phi_slot(int ti, int tj, int nt) {
@@ -751,6 +755,21 @@ __device__ __forceinline__ void ld_rows2(const float4* p, float4& a, float4& b) 
   asm volatile("ld.global.nc.L1::evict_last.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
       : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
       : "l"(p));
+}
+
+// The derivative coefficients of one single-type FP64 bin from the two split
+// arrays (the value slots stay unset).  A warp's 32 random bins cost 29 L1
+// cycles this way, 49 as two 32-byte rows 64 bytes apart (which use half of
+// the banks each), 32 as three 16-byte loads; the pass is bound by L1: EAM 131k
+// FP64 6.47 -> 5.75 ms per 50 steps.
+template <class T>
+__device__ __forceinline__ void ld_derivs(const EamDev<T>& e, int idx, double4& rho,
+                                          double4& phi) {
+  rho = ld_d4(e.d4 + idx);
+  phi.x = rho.w;
+  asm volatile("ld.global.nc.L1::evict_last.v2.f64 {%0, %1}, [%2];"
+      : "=d"(phi.y), "=d"(phi.z)
+      : "l"(e.d2 + idx));
 }
 
 // Embedding F(rho), F'(rho) in FP64 (SplineTable eval/eval_deriv on F).
@@ -965,6 +984,8 @@ __global__ void __launch_bounds__(256) k_eam_force(Geo g, NbrView nl, int n,
           typename V4<T>::type cphi, crho;
           if constexpr (!MULTI && sizeof(T) == sizeof(float)) {
             ld_rows2(rowp, crho, cphi);  // single type: S = 2, slots rho', phi'
+          } else if constexpr (!MULTI && EV == 0) {
+            ld_derivs(e, idx, crho, cphi);
           } else {
             cphi = ldv4<T>(rowp + (MULTI ? phi_slot(ti, tj, e.ntypes) : 1));
             crho = ldv4<T>(rowp + tj);
