@@ -27,8 +27,8 @@
 // per step.  Gradients accumulate in FP64 (per-block partials for the three
 // Morse parameters; FP64 atomics into the coefficient arrays for EAM).
 // Passes: Morse = forces+G, gradient; EAM = density (+F', F''), forces+G,
-// adjoint (phi / rho-derivative / F terms and w_i, then the rho-value term
-// in a second sweep of the same atom's row).
+// adjoint weights w_i (+ F terms), then the phi and rho terms over the
+// unordered pairs.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -47,51 +47,36 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kPart = 4;  // doubles per block partial
 
-// Packed spline coefficients a|b|c|d (SplineTable::build_splines layout,
-// eam_alloy.cpp:19-50), one spline of ns intervals at `c`.
-struct SplC {
-  const double* c;
-  int ns;
-  double step;
-};
-
-__device__ __forceinline__ int spl_seg(double x, double step, int ns, double& dx) {
-  return spline_idx(x, step, ns + 1, dx);
-}
-
+// One row (a, b, c, d) per spline interval, so that a pair's lookup is one
+// 32-byte load per spline (the packed a|b|c|d arrays the caller passes take
+// four 8-byte gathers: 33 L1 cycles for a warp's random intervals, 19 for one
+// row).
 template <class T>
-__device__ __forceinline__ T spl_value(const SplC& s, int k, T dx) {
-  const T a = static_cast<T>(__ldg(s.c + k)), b = static_cast<T>(__ldg(s.c + s.ns + k));
-  const T c = static_cast<T>(__ldg(s.c + 2 * s.ns + k)),
-          d = static_cast<T>(__ldg(s.c + 3 * s.ns + k));
+__device__ __forceinline__ T row_value(const double4& r, T dx) {
+  const T a = static_cast<T>(r.x), b = static_cast<T>(r.y), c = static_cast<T>(r.z),
+          d = static_cast<T>(r.w);
   return a + dx * (b + dx * (c + dx * d));
 }
-
 template <class T>
-__device__ __forceinline__ T spl_deriv(const SplC& s, int k, T dx) {
-  const T b = static_cast<T>(__ldg(s.c + s.ns + k));
-  const T c = static_cast<T>(__ldg(s.c + 2 * s.ns + k)),
-          d = static_cast<T>(__ldg(s.c + 3 * s.ns + k));
+__device__ __forceinline__ T row_deriv(const double4& r, T dx) {
+  const T b = static_cast<T>(r.y), c = static_cast<T>(r.z), d = static_cast<T>(r.w);
   return b + dx * (T(2) * c + T(3) * d * dx);
 }
 
-// 1/r as a double: the FP64 geometries' own, a division of the FP32 radius.
-__device__ __forceinline__ double inv_radius(double /*r*/, double rinv) { return rinv; }
-__device__ __forceinline__ double inv_radius(float r, float /*rinv*/) {
-  return 1.0 / static_cast<double>(r);
+// Gradient of an interval's coefficients in a packed a|b|c|d array: wd times
+// the derivative's basis (0, 1, 2x, 3x^2) plus wv times the value's
+// (1, x, x^2, x^3).
+__device__ __forceinline__ void add_deriv_basis(double* g, int ns, int k, double dx, double wd) {
+  atomicAdd(g + ns + k, wd);
+  atomicAdd(g + 2 * ns + k, 2.0 * wd * dx);
+  atomicAdd(g + 3 * ns + k, 3.0 * wd * dx * dx);
 }
-
-// Gradient scatter into a packed a|b|c|d spline gradient.
-__device__ __forceinline__ void add_value_basis(double* g, int ns, int k, double dx, double w) {
-  atomicAdd(g + k, w);
-  atomicAdd(g + ns + k, w * dx);
-  atomicAdd(g + 2 * ns + k, w * dx * dx);
-  atomicAdd(g + 3 * ns + k, w * dx * dx * dx);
-}
-__device__ __forceinline__ void add_deriv_basis(double* g, int ns, int k, double dx, double w) {
-  atomicAdd(g + ns + k, w);
-  atomicAdd(g + 2 * ns + k, 2.0 * w * dx);
-  atomicAdd(g + 3 * ns + k, 3.0 * w * dx * dx);
+__device__ __forceinline__ void add_both_bases(double* g, int ns, int k, double dx, double wd,
+                                               double wv) {
+  atomicAdd(g + k, wv);
+  atomicAdd(g + ns + k, fma(wv, dx, wd));
+  atomicAdd(g + 2 * ns + k, dx * fma(wv, dx, 2.0 * wd));
+  atomicAdd(g + 3 * ns + k, dx * dx * fma(wv, dx, 3.0 * wd));
 }
 
 __device__ __forceinline__ int pair_index(int ti, int tj, int nt) {
@@ -103,25 +88,32 @@ __device__ __forceinline__ int pair_index(int ti, int tj, int nt) {
   return ti * nt - ti * (ti + 1) / 2 + tj;
 }
 
-// Device view of the EAM coefficient arrays being fitted and their
-// gradients (types 0-based here).
+// Device view of the EAM coefficient arrays being fitted, the row copies the
+// passes read and the gradients (types 0-based here).
 struct FitEam {
   const double* F;
-  const double* rho;
-  const double* phi;
+  const double4* rows;  // [nt + npairs][nsr]: rho_t, then phi_p
   double* gF;
   double* grho;
   double* gphi;
   int nt, nsf, nsr;
   double drho, dr, inv_dr;
-  __device__ __forceinline__ SplC Fs(int t) const { return SplC{F + 4ll * nsf * t, nsf, drho}; }
-  __device__ __forceinline__ SplC rhos(int t) const {
-    return SplC{rho + 4ll * nsr * t, nsr, dr};
+  __device__ __forceinline__ double4 rho_row(int t, int k) const {
+    return ld_d4(rows + static_cast<long long>(t) * nsr + k);
   }
-  __device__ __forceinline__ SplC phis(int p) const {
-    return SplC{phi + 4ll * nsr * p, nsr, dr};
+  __device__ __forceinline__ double4 phi_row(int p, int k) const {
+    return ld_d4(rows + static_cast<long long>(nt + p) * nsr + k);
+  }
+  __device__ __forceinline__ int seg(double r, double& dx) const {
+    return spline_idx_mul(r, dr, inv_dr, nsr + 1, dx);
   }
 };
+
+// 1/r as a double: the FP64 geometries' own, a division of the FP32 radius.
+__device__ __forceinline__ double inv_radius(double /*r*/, double rinv) { return rinv; }
+__device__ __forceinline__ double inv_radius(float r, float /*rinv*/) {
+  return 1.0 / static_cast<double>(r);
+}
 
 // Block partial sums: lane merge -> warp -> block; thread 0 writes kPart.
 template <int NV>
@@ -141,13 +133,33 @@ __device__ __forceinline__ T lane_sum(T v) {
   return v;
 }
 
+// Atom i's share of the loss; G_i = dL/dF_i goes out with w in the record's
+// fourth word.
+__device__ __forceinline__ double residual(double fx, double fy, double fz,
+                                           const double* __restrict__ target, double c, int i,
+                                           double w, double4* __restrict__ G,
+                                           double* __restrict__ fout) {
+  const double ex = fx - target[3ll * i], ey = fy - target[3ll * i + 1],
+               ez = fz - target[3ll * i + 2];
+  G[i] = make_double4(2.0 * c * ex, 2.0 * c * ey, 2.0 * c * ez, w);
+  if (fout) {
+    fout[3ll * i] = fx;
+    fout[3ll * i + 1] = fy;
+    fout[3ll * i + 2] = fz;
+  }
+  double v = c * ex * ex;
+  v += c * ey * ey;
+  v += c * ez * ez;
+  return v;
+}
+
 // ---------------------------------------------------------------------------
 // Morse
 // ---------------------------------------------------------------------------
 template <class Geo, int LPA>
 __global__ void __launch_bounds__(kThreads) k_fm_morse_force(
     Geo g, NbrView nl, int n, const double* __restrict__ prm, double rc_sq,
-    const double* __restrict__ target, double c, double* __restrict__ G,
+    const double* __restrict__ target, double c, double4* __restrict__ G,
     double* __restrict__ fout, double* __restrict__ part) {
   dependent_launch_prologue();
   using T = typename Geo::T;
@@ -184,13 +196,7 @@ __global__ void __launch_bounds__(kThreads) k_fm_morse_force(
   }
   double v[1] = {0.0};
   if (active && sub == 0) {
-    const double f[3] = {fx.value(), fy.value(), fz.value()};
-    for (int a = 0; a < 3; ++a) {
-      const double e = f[a] - target[3ll * i + a];
-      v[0] += c * e * e;
-      G[3ll * i + a] = 2.0 * c * e;
-      if (fout) fout[3ll * i + a] = f[a];
-    }
+    v[0] = residual(fx.value(), fy.value(), fz.value(), target, c, i, 0.0, G, fout);
   }
   write_partials<1>(v, part);
 }
@@ -199,7 +205,7 @@ template <class Geo, int LPA>
 __global__ void __launch_bounds__(kThreads) k_fm_morse_grad(Geo g, NbrView nl, int n,
                                                             const double* __restrict__ prm,
                                                             double rc_sq,
-                                                            const double* __restrict__ G,
+                                                            const double4* __restrict__ G,
                                                             double* __restrict__ part) {
   dependent_launch_prologue();
   using T = typename Geo::T;
@@ -210,7 +216,7 @@ __global__ void __launch_bounds__(kThreads) k_fm_morse_grad(Geo g, NbrView nl, i
   double v[3] = {0.0, 0.0, 0.0};
   if (i < n) {
     const typename Geo::Own o = g.own(i);
-    const double gx = G[3ll * i], gy = G[3ll * i + 1], gz = G[3ll * i + 2];
+    const double4 gi = G[i];
     const long long row = nl.row(i);
     const int cnt = nl.count(i);
     for (int k = sub; k < cnt; k += LPA) {
@@ -222,8 +228,9 @@ __global__ void __launch_bounds__(kThreads) k_fm_morse_grad(Geo g, NbrView nl, i
         g.radius(o, pr, r, rinv, rd);
         const T ex = exp(-at * static_cast<T>(rd - r0));
         const T ome = T(1) - ex;
-        const double gd = (gx * static_cast<double>(pr.dx) + gy * static_cast<double>(pr.dy) +
-                           gz * static_cast<double>(pr.dz)) * inv_radius(r, rinv);
+        const double gd = (gi.x * static_cast<double>(pr.dx) + gi.y * static_cast<double>(pr.dy) +
+                           gi.z * static_cast<double>(pr.dz)) *
+                          inv_radius(r, rinv);
         // df/dtheta * r (the 1/r is folded into gd)
         const T dD = -T(2) * at * ome * ex;
         const T da = -T(2) * Dt * (ome * ex - at * (T(1) - T(2) * ex) *
@@ -239,10 +246,16 @@ __global__ void __launch_bounds__(kThreads) k_fm_morse_grad(Geo g, NbrView nl, i
 }
 
 // Sums nblk block partials (kPart doubles each) in block order:
-// out[0..nv) = column sums.
-__global__ void k_fm_sum(const double* __restrict__ part, int nblk, int nv,
-                         double* __restrict__ out) {
+// out[0..nv) = column sums; a second block does the same for part2 / out2.
+__global__ void k_fm_sum(const double* __restrict__ part, int nv, double* __restrict__ out,
+                         const double* __restrict__ part2, int nv2, double* __restrict__ out2,
+                         int nblk) {
   dependent_launch_prologue();
+  if (blockIdx.x == 1) {
+    part = part2;
+    nv = nv2;
+    out = out2;
+  }
   __shared__ double red[32 * kPart];
   double v[kPart] = {0.0, 0.0, 0.0, 0.0};
   for (int b = threadIdx.x; b < nblk; b += blockDim.x)
@@ -255,18 +268,41 @@ __global__ void k_fm_sum(const double* __restrict__ part, int nblk, int nv,
 // ---------------------------------------------------------------------------
 // EAM
 // ---------------------------------------------------------------------------
+// Row copies of the r splines and zeroed gradients, before the passes.
+__global__ void k_fm_rows(const double* __restrict__ rho, const double* __restrict__ phi, int nt,
+                          int np, int nsr, double4* __restrict__ rows, double* __restrict__ gF,
+                          long long nF, double* __restrict__ grho, double* __restrict__ gphi) {
+  dependent_launch_prologue();
+  const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
+  const long long nr = static_cast<long long>(nt) * nsr, n = nr + static_cast<long long>(np) * nsr;
+  for (long long q = tid; q < n; q += step) {
+    const long long w = q < nr ? q : q - nr;  // within rho or phi
+    const double* c = (q < nr ? rho : phi) + 4 * nsr * (w / nsr) + w % nsr;
+    rows[q] = make_double4(c[0], c[nsr], c[2 * nsr], c[3 * nsr]);
+  }
+  if (!gF) return;
+  for (long long q = tid; q < nF; q += step) gF[q] = 0.0;
+  for (long long q = tid; q < 4 * nr; q += step) grho[q] = 0.0;
+  for (long long q = tid; q < 4 * (n - nr); q += step) gphi[q] = 0.0;
+}
+
+// rho_i, then F' and F''; the force pass's gather records {position, F'}.
 template <class Geo, int LPA>
 __global__ void __launch_bounds__(kThreads) k_fm_eam_density(
     Geo g, NbrView nl, int n, const int* __restrict__ types, FitEam e, double rc_sq,
-    double* __restrict__ rho_out, double* __restrict__ fp_out, double* __restrict__ fpp_out) {
+    double* __restrict__ rho_out, double* __restrict__ fp_out, double* __restrict__ fpp_out,
+    double4* __restrict__ rec_d, int4* __restrict__ rec_q) {
   dependent_launch_prologue();
   using T = typename Geo::T;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = tid / LPA, sub = tid % LPA;
   const bool active = i < n;
+  const bool multi = e.nt > 1;
   Acc<T> rho;
+  typename Geo::Own o{};
   if (active) {
-    const typename Geo::Own o = g.own(i);
+    o = g.own(i);
     const long long row = nl.row(i);
     const int cnt = nl.count(i);
     for (int k = sub; k < cnt; k += LPA) {
@@ -278,8 +314,9 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_density(
         double rd;
         g.radius(o, pr, r, rinv, rd);
         double dx;
-        const int kk = spline_idx_mul(rd, e.dr, e.inv_dr, e.nsr + 1, dx);
-        rho.add(spl_value<T>(e.rhos(__ldg(types + j) - 1), kk, static_cast<T>(dx)));
+        const int kk = e.seg(rd, dx);
+        const int tj = multi ? __ldg(types + j) - 1 : 0;
+        rho.add(row_value<T>(e.rho_row(tj, kk), static_cast<T>(dx)));
       }
     }
   }
@@ -287,29 +324,41 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_density(
   for (int s = LPA / 2; s > 0; s >>= 1) rho.shfl_merge(s);
   if (active && sub == 0) {
     const double rh = rho.value();
-    const SplC F = e.Fs(__ldg(types + i) - 1);
+    const double* F = e.F + 4ll * e.nsf * (multi ? __ldg(types + i) - 1 : 0);
     double dx;
-    const int kk = spl_seg(rh, e.drho, e.nsf, dx);
+    const int kk = spline_idx(rh, e.drho, e.nsf + 1, dx);
+    const double b = __ldg(F + e.nsf + kk), c = __ldg(F + 2 * e.nsf + kk),
+                 d = __ldg(F + 3 * e.nsf + kk);
+    const double fp = b + dx * (2.0 * c + 3.0 * d * dx);
     rho_out[i] = rh;
-    fp_out[i] = spl_deriv<double>(F, kk, dx);
-    fpp_out[i] = 2.0 * __ldg(F.c + 2 * F.ns + kk) + 6.0 * __ldg(F.c + 3 * F.ns + kk) * dx;
+    fp_out[i] = fp;
+    fpp_out[i] = 2.0 * c + 6.0 * d * dx;
+    if constexpr (Geo::kRecords) {
+      int4 rec = g.record(o);
+      rec.w = __float_as_int(static_cast<float>(fp));
+      rec_q[i] = rec;
+    } else {
+      rec_d[i] = make_double4(o.x, o.y, o.z, fp);
+    }
   }
 }
 
+// Forces from the {position, F'} records, residuals, G.
 template <class Geo, int LPA>
 __global__ void __launch_bounds__(kThreads) k_fm_eam_force(
     Geo g, NbrView nl, int n, const int* __restrict__ types, FitEam e, double rc_sq,
     const double* __restrict__ fp, const double* __restrict__ target, double c,
-    double* __restrict__ G, double* __restrict__ fout, double* __restrict__ part) {
+    double4* __restrict__ G, double* __restrict__ fout, double* __restrict__ part) {
   dependent_launch_prologue();
   using T = typename Geo::T;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = tid / LPA, sub = tid % LPA;
   const bool active = i < n;
+  const bool multi = e.nt > 1;
   Acc<T> fx, fy, fz;
   if (active) {
     const typename Geo::Own o = g.own(i);
-    const int ti = __ldg(types + i) - 1;
+    const int ti = multi ? __ldg(types + i) - 1 : 0;
     const T fpi = static_cast<T>(fp[i]);
     const long long row = nl.row(i);
     const int cnt = nl.count(i);
@@ -321,14 +370,14 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_force(
         T r, rinv;
         double rd;
         g.radius(o, pr, r, rinv, rd);
-        const int tj = __ldg(types + j) - 1;
+        const int tj = multi ? __ldg(types + j) - 1 : 0;
         double dxd;
-        const int kk = spline_idx_mul(rd, e.dr, e.inv_dr, e.nsr + 1, dxd);
+        const int kk = e.seg(rd, dxd);
         const T dx = static_cast<T>(dxd);
-        const T dphi = spl_deriv<T>(e.phis(pair_index(ti, tj, e.nt)), kk, dx);
-        const T drj = spl_deriv<T>(e.rhos(tj), kk, dx);
-        const T dri = ti == tj ? drj : spl_deriv<T>(e.rhos(ti), kk, dx);
-        const T fpair = -div_r(dphi + fpi * drj + static_cast<T>(fp[j]) * dri, r, rinv);
+        const T dphi = row_deriv<T>(e.phi_row(multi ? pair_index(ti, tj, e.nt) : 0, kk), dx);
+        const T drj = row_deriv<T>(e.rho_row(tj, kk), dx);
+        const T dri = ti == tj ? drj : row_deriv<T>(e.rho_row(ti, kk), dx);
+        const T fpair = -div_r(dphi + fpi * drj + static_cast<T>(g.gather_fp(pr, 0)) * dri, r, rinv);
         fx.add(mul_rn(fpair, pr.dx));
         fy.add(mul_rn(fpair, pr.dy));
         fz.add(mul_rn(fpair, pr.dz));
@@ -342,204 +391,203 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_force(
     fz.shfl_merge(s);
   }
   double v[1] = {0.0};
-  if (active && sub == 0) {
-    const double f[3] = {fx.value(), fy.value(), fz.value()};
-    for (int a = 0; a < 3; ++a) {
-      const double d = f[a] - target[3ll * i + a];
-      v[0] += c * d * d;
-      G[3ll * i + a] = 2.0 * c * d;
-      if (fout) fout[3ll * i + a] = f[a];
-    }
-  }
+  if (active && sub == 0)
+    v[0] = residual(fx.value(), fy.value(), fz.value(), target, c, i, fp[i], G, fout);
   write_partials<1>(v, part);
 }
 
+// Adjoint, first pass: w_i over atom i's row, the F coefficients' gradient,
+// and wf_i = w_i F''_i for the second pass.
 template <class Geo, int LPA>
-__global__ void __launch_bounds__(kThreads) k_fm_eam_adjoint(
+__global__ void __launch_bounds__(kThreads) k_fm_eam_weights(
     Geo g, NbrView nl, int n, const int* __restrict__ types, FitEam e, double rc_sq,
-    const double* __restrict__ rho, const double* __restrict__ fp,
-    const double* __restrict__ fpp, const double* __restrict__ G) {
+    const double* __restrict__ rho, const double* __restrict__ fpp,
+    const double4* __restrict__ G, double* __restrict__ wf) {
   dependent_launch_prologue();
   using T = typename Geo::T;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = tid / LPA, sub = tid % LPA;
   const bool active = i < n;
+  const bool multi = e.nt > 1;
   double w = 0.0;
-  typename Geo::Own o{};
-  int ti = 0, cnt = 0;
-  long long row = 0;
   if (active) {
-    o = g.own(i);
-    ti = __ldg(types + i) - 1;
-    row = nl.row(i);
-    cnt = nl.count(i);
-    const double gix = G[3ll * i], giy = G[3ll * i + 1], giz = G[3ll * i + 2];
-    const double fpi = fp[i];
+    const typename Geo::Own o = g.own(i);
+    const double4 gi = G[i];
+    const long long row = nl.row(i);
+    const int cnt = nl.count(i);
     for (int k = sub; k < cnt; k += LPA) {
       const int j = __ldg(nl.nbr + row + k);
       typename Geo::Pair pr;
       g.pair(o, j, pr);
       if (pr.r2 < static_cast<T>(rc_sq)) {
+        const double4 gj = ld_d4(G + j);
         T r, rinv;
         double rd;
         g.radius(o, pr, r, rinv, rd);
-        const int tj = __ldg(types + j) - 1;
         double dx;
-        const int kk = spline_idx_mul(rd, e.dr, e.inv_dr, e.nsr + 1, dx);
-        const double ddx = pr.dx, ddy = pr.dy, ddz = pr.dz, ri = inv_radius(r, rinv);
-        const double q = (gix * ddx + giy * ddy + giz * ddz) * ri;
-        const double fpj = fp[j];
-        add_deriv_basis(e.gphi + 4ll * e.nsr * pair_index(ti, tj, e.nt), e.nsr, kk, dx, -q);
-        if (ti == tj) {
-          add_deriv_basis(e.grho + 4ll * e.nsr * tj, e.nsr, kk, dx, -q * (fpi + fpj));
-        } else {
-          add_deriv_basis(e.grho + 4ll * e.nsr * tj, e.nsr, kk, dx, -q * fpi);
-          add_deriv_basis(e.grho + 4ll * e.nsr * ti, e.nsr, kk, dx, -q * fpj);
-        }
-        const double drj = spl_deriv<double>(e.rhos(tj), kk, dx);
-        const double gdiff = (gix - G[3ll * j]) * ddx + (giy - G[3ll * j + 1]) * ddy +
-                             (giz - G[3ll * j + 2]) * ddz;
-        w -= drj * gdiff * ri;
+        const int kk = e.seg(rd, dx);
+        const double dr = row_deriv<double>(e.rho_row(multi ? __ldg(types + j) - 1 : 0, kk), dx);
+        const double gd = (gi.x - gj.x) * static_cast<double>(pr.dx) +
+                          (gi.y - gj.y) * static_cast<double>(pr.dy) +
+                          (gi.z - gj.z) * static_cast<double>(pr.dz);
+        w -= dr * gd * inv_radius(r, rinv);
       }
     }
   }
   w = lane_sum<double, LPA>(w);
-  if (!active) return;
-  if (sub == 0) {
+  if (active && sub == 0) {
     double dx;
-    const int kk = spl_seg(rho[i], e.drho, e.nsf, dx);
-    add_deriv_basis(e.gF + 4ll * e.nsf * ti, e.nsf, kk, dx, w);
-  }
-  const double wf = w * fpp[i];
-  // rho values through rho_i: w_i F''_i * drho_tj/dc at r_ij.
-  for (int k = sub; k < cnt; k += LPA) {
-    const int j = __ldg(nl.nbr + row + k);
-    typename Geo::Pair pr;
-    g.pair(o, j, pr);
-    if (pr.r2 < static_cast<T>(rc_sq)) {
-      T r, rinv;
-      double rd;
-      g.radius(o, pr, r, rinv, rd);
-      const int tj = __ldg(types + j) - 1;
-      double dx;
-      const int kk = spline_idx_mul(rd, e.dr, e.inv_dr, e.nsr + 1, dx);
-      add_value_basis(e.grho + 4ll * e.nsr * tj, e.nsr, kk, dx, wf);
-    }
+    const int kk = spline_idx(rho[i], e.drho, e.nsf + 1, dx);
+    add_deriv_basis(e.gF + 4ll * e.nsf * (multi ? __ldg(types + i) - 1 : 0), e.nsf, kk, dx, w);
+    wf[i] = w * fpp[i];
   }
 }
 
-// Single-element alloys: the same adjoint with the r-spline gradients
-// (phi, rho) of intervals [k0, k0 + W) accumulated in shared memory by each
-// block of a persistent grid and added to the global arrays once per block
-// at the end; intervals below k0 (pairs closer than k0 * dr) go straight to
-// global memory.  Shared layout: [phi, rho][coefficient 0..3][W].
-__device__ __forceinline__ void add_r(double* gl, double* sh, int ns, int k, int k0, int W,
-                                      int coef, double v) {
-  if (k >= k0) atomicAdd(sh + coef * W + (k - k0), v);
-  else atomicAdd(gl + coef * ns + k, v);
-}
-
-template <class Geo, int LPA>
-__global__ void __launch_bounds__(kThreads) k_fm_eam_adjoint_w(
-    Geo g, NbrView nl, int n, FitEam e, double rc_sq, const double* __restrict__ rho,
-    const double* __restrict__ fp, const double* __restrict__ fpp,
-    const double* __restrict__ G, int k0, int W) {
+// Adjoint, second pass: the phi and rho coefficients, each unordered pair
+// once.  The ordered pairs (i, j) and (j, i) meet the same intervals with
+// weights that add up: with q = (G_i - G_j) . d / r,
+//   phi_p   derivative -q;
+//   rho_tj  derivative -q F'_i, value w_i F''_i;
+//   rho_ti  derivative -q F'_j, value w_j F''_j
+// (one type: one rho spline with both sums), so an unordered pair takes 3 + 4
+// scattered adds for one type where the two ordered pairs took 20.  The pass
+// is bound by those adds (0.81 cycles per lane and SM in shared memory, 2.1
+// in L2).  69 984 atoms, 1.5 M pairs: loss and gradient 280 -> 196 us, of
+// which the one-sweep adjoint over ordered pairs took 178.
+//
+// SHARED (one type): the adds to intervals [k0, k0 + W) go to shared memory,
+// one block of 1024 threads per SM over a persistent grid, and out once as a
+// block partial ([7][W] doubles, summed by k_fm_eam_window): 148 blocks
+// adding their 1 280 x 7 sums to global memory instead took 10 us more.
+// Intervals below k0 (pairs closer than k0 * dr) go straight to global
+// memory, as every interval does for several types.
+constexpr int kPairThreads = 1024;
+template <class Geo, int LPA, bool SHARED>
+__global__ void __launch_bounds__(SHARED ? kPairThreads : kThreads) k_fm_eam_pairs(
+    Geo g, NbrView nl, int n, const int* __restrict__ types, FitEam e, double rc_sq,
+    const double4* __restrict__ G, const double* __restrict__ wf, int k0, int W,
+    double* __restrict__ part) {
   dependent_launch_prologue();
   using T = typename Geo::T;
   extern __shared__ double sg[];
-  double* const sphi = sg;
-  double* const srho = sg + 4 * W;
-  for (int k = threadIdx.x; k < 8 * W; k += blockDim.x) sg[k] = 0.0;
-  __syncthreads();
+  if (SHARED) {
+    for (int k = threadIdx.x; k < 7 * W; k += blockDim.x) sg[k] = 0.0;
+    __syncthreads();
+  }
   const int ns = e.nsr;
   const int per_block = blockDim.x / LPA;
   const int sub = threadIdx.x % LPA;
-  for (long long first = static_cast<long long>(blockIdx.x) * per_block; first < n;
-       first += static_cast<long long>(gridDim.x) * per_block) {
-    const long long ii = first + threadIdx.x / LPA;
-    const bool active = ii < n;
-    const int i = active ? static_cast<int>(ii) : 0;
-    double w = 0.0;
-    typename Geo::Own o{};
-    int cnt = 0;
-    long long row = 0;
-    if (active) {
-      o = g.own(i);
-      row = nl.row(i);
-      cnt = nl.count(i);
-      const double gix = G[3ll * i], giy = G[3ll * i + 1], giz = G[3ll * i + 2];
-      const double fpi = fp[i];
-      for (int k = sub; k < cnt; k += LPA) {
-        const int j = __ldg(nl.nbr + row + k);
-        typename Geo::Pair pr;
-        g.pair(o, j, pr);
-        if (pr.r2 < static_cast<T>(rc_sq)) {
-          T r, rinv;
-          double rd;
-          g.radius(o, pr, r, rinv, rd);
-          double dx;
-          const int kk = spline_idx_mul(rd, e.dr, e.inv_dr, ns + 1, dx);
-          const double ddx = pr.dx, ddy = pr.dy, ddz = pr.dz, ri = inv_radius(r, rinv);
-          const double q = (gix * ddx + giy * ddy + giz * ddz) * ri;
-          const double fpj = fp[j];
-          // phi' and rho' terms: d/dc of the derivative basis (b, 2c x, 3d x^2)
-          const double wp = -q, wr = -q * (fpi + fpj);
-          add_r(e.gphi, sphi, ns, kk, k0, W, 1, wp);
-          add_r(e.gphi, sphi, ns, kk, k0, W, 2, 2.0 * wp * dx);
-          add_r(e.gphi, sphi, ns, kk, k0, W, 3, 3.0 * wp * dx * dx);
-          add_r(e.grho, srho, ns, kk, k0, W, 1, wr);
-          add_r(e.grho, srho, ns, kk, k0, W, 2, 2.0 * wr * dx);
-          add_r(e.grho, srho, ns, kk, k0, W, 3, 3.0 * wr * dx * dx);
-          const double drj = spl_deriv<double>(e.rhos(0), kk, dx);
-          const double gdiff = (gix - G[3ll * j]) * ddx + (giy - G[3ll * j + 1]) * ddy +
-                               (giz - G[3ll * j + 2]) * ddz;
-          w -= drj * gdiff * ri;
-        }
-      }
-    }
-    w = lane_sum<double, LPA>(w);
-    if (active) {
-      if (sub == 0) {
-        double dx;
-        const int kk = spl_seg(rho[i], e.drho, e.nsf, dx);
-        add_deriv_basis(e.gF, e.nsf, kk, dx, w);
-      }
-      const double wf = w * fpp[i];
-      // rho values through rho_i: w_i F''_i * drho/dc at r_ij
-      for (int k = sub; k < cnt; k += LPA) {
-        const int j = __ldg(nl.nbr + row + k);
-        typename Geo::Pair pr;
-        g.pair(o, j, pr);
-        if (pr.r2 < static_cast<T>(rc_sq)) {
-          T r, rinv;
-          double rd;
-          g.radius(o, pr, r, rinv, rd);
-          double dx;
-          const int kk = spline_idx_mul(rd, e.dr, e.inv_dr, ns + 1, dx);
-          add_r(e.grho, srho, ns, kk, k0, W, 0, wf);
-          add_r(e.grho, srho, ns, kk, k0, W, 1, wf * dx);
-          add_r(e.grho, srho, ns, kk, k0, W, 2, wf * dx * dx);
-          add_r(e.grho, srho, ns, kk, k0, W, 3, wf * dx * dx * dx);
+  for (long long ii = static_cast<long long>(blockIdx.x) * per_block + threadIdx.x / LPA; ii < n;
+       ii += static_cast<long long>(gridDim.x) * per_block) {
+    const int i = static_cast<int>(ii);
+    const typename Geo::Own o = g.own(i);
+    const double4 gi = G[i];
+    const double wi = wf[i];
+    const int ti = SHARED ? 0 : __ldg(types + i) - 1;
+    const long long row = nl.row(i);
+    const int cnt = nl.count(i);
+    for (int k = sub; k < cnt; k += LPA) {
+      const int j = __ldg(nl.nbr + row + k);
+      if (j < i) continue;
+      typename Geo::Pair pr;
+      g.pair(o, j, pr);
+      if (!(pr.r2 < static_cast<T>(rc_sq))) continue;
+      const double4 gj = ld_d4(G + j);
+      const double wj = __ldg(wf + j);
+      T r, rinv;
+      double rd;
+      g.radius(o, pr, r, rinv, rd);
+      double dx;
+      const int kk = e.seg(rd, dx);
+      const double q = ((gi.x - gj.x) * static_cast<double>(pr.dx) +
+                        (gi.y - gj.y) * static_cast<double>(pr.dy) +
+                        (gi.z - gj.z) * static_cast<double>(pr.dz)) *
+                       inv_radius(r, rinv);
+      if (SHARED && kk >= k0) {
+        const double wd = -q * (gi.w + gj.w), wv = wi + wj;
+        double* const s = sg + (kk - k0);
+        atomicAdd(s, -q);
+        atomicAdd(s + W, -2.0 * q * dx);
+        atomicAdd(s + 2 * W, -3.0 * q * dx * dx);
+        atomicAdd(s + 3 * W, wv);
+        atomicAdd(s + 4 * W, fma(wv, dx, wd));
+        atomicAdd(s + 5 * W, dx * fma(wv, dx, 2.0 * wd));
+        atomicAdd(s + 6 * W, dx * dx * fma(wv, dx, 3.0 * wd));
+      } else {
+        const int tj = SHARED ? 0 : __ldg(types + j) - 1;
+        add_deriv_basis(e.gphi + 4ll * ns * (SHARED ? 0 : pair_index(ti, tj, e.nt)), ns, kk, dx,
+                        -q);
+        if (ti == tj) {
+          add_both_bases(e.grho + 4ll * ns * tj, ns, kk, dx, -q * (gi.w + gj.w), wi + wj);
+        } else {
+          add_both_bases(e.grho + 4ll * ns * tj, ns, kk, dx, -q * gi.w, wi);
+          add_both_bases(e.grho + 4ll * ns * ti, ns, kk, dx, -q * gj.w, wj);
         }
       }
     }
   }
+  if (SHARED) {
+    __syncthreads();
+    double* const o = part + static_cast<long long>(blockIdx.x) * 7 * W;
+    for (int k = threadIdx.x; k < 7 * W; k += blockDim.x) o[k] = sg[k];
+  }
+}
+
+// Adds the block partials of k_fm_eam_pairs to the gradients: 32 columns of
+// the 7 W per block, 8 threads sharing a column's nblk records.
+__global__ void __launch_bounds__(256) k_fm_eam_window(const double* __restrict__ part, int nblk,
+                                                       int W, int k0, int ns,
+                                                       double* __restrict__ gphi,
+                                                       double* __restrict__ grho) {
+  dependent_launch_prologue();
+  __shared__ double red[8][32];
+  const int c = blockIdx.x * 32 + (threadIdx.x & 31), part_of = threadIdx.x >> 5;
+  double v = 0.0;
+  if (c < 7 * W) {
+#pragma unroll 4
+    for (int b = part_of; b < nblk; b += 8) v += part[static_cast<long long>(b) * 7 * W + c];
+  }
+  red[part_of][threadIdx.x & 31] = v;
   __syncthreads();
-  for (int k = threadIdx.x; k < 8 * W; k += blockDim.x) {
-    const double v = sg[k];
-    if (v != 0.0) {
-      const int sp = k / (4 * W), coef = (k / W) % 4, b = k % W;
-      atomicAdd((sp == 0 ? e.gphi : e.grho) + coef * ns + k0 + b, v);
-    }
+  if (part_of == 0 && c < 7 * W) {
+    for (int k = 1; k < 8; ++k) v += red[k][threadIdx.x];
+    const int coef = c / W, k = k0 + c % W;
+    // columns: phi's b, c, d, then rho's a, b, c, d
+    double* const g = coef < 3 ? gphi + (coef + 1) * ns + k : grho + (coef - 3) * ns + k;
+    *g += v;
   }
 }
 
 }  // namespace
 
 // Intervals of the r splines whose gradients a block keeps in shared memory
-// (8 doubles each: 4 coefficients of phi and of rho): 1280 x 64 B = 80 KiB,
-// two blocks per SM.
+// (7 doubles each): the top 1280, 70 KiB.
 constexpr int kAdjointWindow = 1280;
+
+// The spline rows of one call: the handle's buffer, except while the stream is
+// captured, when they belong to the graph (a buffer that a later call with
+// larger tables would replace must not be in it).
+struct RowScratch {
+  double4* p = nullptr;
+  cudaStream_t s = nullptr;
+  bool owned = false;
+  RowScratch(DevArray<double4>& keep, size_t n, cudaStream_t st) : s(st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    TDMD_CU(cudaStreamIsCapturing(st, &cs));
+    if (cs == cudaStreamCaptureStatusNone) {
+      keep.reserve(n);
+      p = keep.data();
+    } else {
+      TDMD_CU(cudaMallocAsync(reinterpret_cast<void**>(&p), n * sizeof(double4), st));
+      owned = true;
+    }
+  }
+  ~RowScratch() {
+    if (owned) cudaFreeAsync(p, s);
+  }
+  RowScratch(const RowScratch&) = delete;
+  RowScratch& operator=(const RowScratch&) = delete;
+};
 
 class Fit {
  public:
@@ -579,7 +627,12 @@ class Fit {
   DevArray<int4> q_;
   DevArray<int> types_;
   DevArray<int> nbr_, cnt_, status_;
-  DevArray<double> target_, G_, rho_, fp_, fpp_, part_;
+  DevArray<double> target_, rho_, fp_, fpp_, wf_, part_;
+  DevArray<double4> G_;      // {dL/dF_i, F'_i}
+  DevArray<double4> rec_;    // FP64 {position, F'} gather records
+  DevArray<int4> recq_;      // mixed: fixed-point position, F' bits
+  DevArray<double4> rows_;   // row copies of the r splines
+  DevArray<double> window_;  // block partials of the shared-memory window
   CellListDev cl_;
 };
 
@@ -644,10 +697,15 @@ Fit::Fit(int nsnap, int natoms, const tdmd_box& box, const double* pos, const in
     cnt_.reserve(m);
     status_.reserve(4);
     target_.reserve(3 * m);
-    G_.reserve(3 * m);
+    G_.reserve(m);
     rho_.reserve(m);
     fp_.reserve(m);
     fpp_.reserve(m);
+    wf_.reserve(m);
+    if (mixed_)
+      recq_.reserve(m);
+    else
+      rec_.reserve(m);
     TDMD_CU(cudaMemcpyAsync(reps_.data(), d.data(), sizeof(RepDesc) * d.size(),
                             cudaMemcpyHostToDevice, s));
     TDMD_CU(cudaMemcpyAsync(scales_.data(), scv.data(), sizeof(RepScale) * scv.size(),
@@ -686,7 +744,10 @@ Fit::Fit(int nsnap, int natoms, const tdmd_box& box, const double* pos, const in
     build_neighbor_rows_batch(cl_, pos4_.data(), reps_.data(), cell_rep_.data(), rc_sq_,
                               nbr_.data(), cap_, cnt_.data(), nullptr, s);
     lpa_ = default_lpa(m_);
-    part_.reserve(static_cast<size_t>(force_blocks(m_, 32)) * kPart + kPart);
+    // the largest window a call can ask for, so that no call allocates it
+    window_.reserve(static_cast<size_t>(std::min(sm_count(), ceil_div(m_ * lpa_, kPairThreads))) *
+                    7 * kAdjointWindow);
+    part_.reserve(2 * (static_cast<size_t>(force_blocks(m_, 32)) * kPart + kPart));
     TDMD_CU(cudaStreamSynchronize(s));
   } catch (...) {
     cudaStreamDestroy(s);
@@ -728,18 +789,19 @@ void Fit::morse(const double* d_prm, double* d_loss, double* d_grad, double* d_f
     });
   });
   TDMD_LAUNCH_CHECK();
-  launch(k_fm_sum, 1, kThreads, 0, s, part_.data(), nblk, 1, d_loss);
-  TDMD_LAUNCH_CHECK();
-  if (!d_grad) return;
-  with_geo([&](auto g) {
-    using Geo = decltype(g);
-    TDMD_LPA_DISPATCH(lpa_, {
-      launch(k_fm_morse_grad<Geo, L>, nblk, kThreads, 0, s, g, nl, m, d_prm, rc_sq_, G_.data(),
-             part_.data());
+  double* const part2 = part_.data() + static_cast<size_t>(nblk) * kPart;
+  if (d_grad) {
+    with_geo([&](auto g) {
+      using Geo = decltype(g);
+      TDMD_LPA_DISPATCH(lpa_, {
+        launch(k_fm_morse_grad<Geo, L>, nblk, kThreads, 0, s, g, nl, m, d_prm, rc_sq_, G_.data(),
+               part2);
+      });
     });
-  });
-  TDMD_LAUNCH_CHECK();
-  launch(k_fm_sum, 1, kThreads, 0, s, part_.data(), nblk, 3, d_grad);
+    TDMD_LAUNCH_CHECK();
+  }
+  launch(k_fm_sum, d_grad ? 2 : 1, kThreads, 0, s, part_.data(), 1, d_loss, part2, 3, d_grad,
+         nblk);
   TDMD_LAUNCH_CHECK();
 }
 
@@ -758,42 +820,54 @@ void Fit::eam(int ntypes, int nrho, double drho, int nr, double dr, const double
   const bool grad = gF || grho || gphi;
   TDMD_REQUIRE(!grad || (gF && grho && gphi), "give all three gradient arrays or none");
   const int npairs = ntypes * (ntypes + 1) / 2;
-  FitEam e{F, rho, phi, gF, grho, gphi, ntypes, nrho - 1, nr - 1, drho, dr, 1.0 / dr};
-  if (grad) {
-    TDMD_CU(cudaMemsetAsync(gF, 0, sizeof(double) * 4 * (nrho - 1) * ntypes, s));
-    TDMD_CU(cudaMemsetAsync(grho, 0, sizeof(double) * 4 * (nr - 1) * ntypes, s));
-    TDMD_CU(cudaMemsetAsync(gphi, 0, sizeof(double) * 4 * (nr - 1) * npairs, s));
-  }
+  const RowScratch rows(rows_, static_cast<size_t>(ntypes + npairs) * (nr - 1), s);
+  const FitEam e{F, rows.p, gF, grho, gphi, ntypes, nrho - 1, nr - 1, drho, dr, 1.0 / dr};
+  launch(k_fm_rows, std::min(2 * sm_count(), ceil_div(4ll * (ntypes + npairs) * (nr - 1), 256)),
+         256, 0, s, rho, phi, ntypes, npairs, nr - 1, rows.p, gF,
+         4ll * (nrho - 1) * ntypes, grho, gphi);
+  TDMD_LAUNCH_CHECK();
   const NbrView nl = view();
   const int m = static_cast<int>(m_);
   const int nblk = force_blocks(m_, lpa_);
   const double c = 1.0 / (3.0 * static_cast<double>(m_));
-  with_geo([&](auto g) {
+  // The window of the shared-memory adjoint (one element).
+  const int W = std::min(nr - 1, kAdjointWindow);
+  const int grid = std::min(sm_count(), ceil_div(m_ * lpa_, kPairThreads));
+  auto passes = [&](auto g, auto gf) {
     using Geo = decltype(g);
+    using GeoF = decltype(gf);
     TDMD_LPA_DISPATCH(lpa_, {
       launch(k_fm_eam_density<Geo, L>, nblk, kThreads, 0, s, g, nl, m, types_.data(), e, rc_sq_,
-             rho_.data(), fp_.data(), fpp_.data());
-      launch(k_fm_eam_force<Geo, L>, nblk, kThreads, 0, s, g, nl, m, types_.data(), e, rc_sq_,
+             rho_.data(), fp_.data(), fpp_.data(), rec_.data(), recq_.data());
+      launch(k_fm_eam_force<GeoF, L>, nblk, kThreads, 0, s, gf, nl, m, types_.data(), e, rc_sq_,
              fp_.data(), target_.data(), c, G_.data(), d_forces, part_.data());
-      if (grad && ntypes == 1) {
-        // one element: shared-memory window of the r-spline gradients over
-        // the top W intervals, a persistent grid of two blocks per SM
-        const int W = std::min(nr - 1, kAdjointWindow);
-        const size_t smem = sizeof(double) * 8 * static_cast<size_t>(W);
-        auto kern = k_fm_eam_adjoint_w<Geo, L>;
-        TDMD_CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem)));
-        const int grid = std::min(2 * sm_count(), nblk);
-        launch(kern, grid, kThreads, smem, s, g, nl, m, e, rc_sq_, rho_.data(), fp_.data(),
-               fpp_.data(), G_.data(), (nr - 1) - W, W);
-      } else if (grad) {
-        launch(k_fm_eam_adjoint<Geo, L>, nblk, kThreads, 0, s, g, nl, m, types_.data(), e, rc_sq_,
-               rho_.data(), fp_.data(), fpp_.data(), G_.data());
+      if (grad) {
+        launch(k_fm_eam_weights<Geo, L>, nblk, kThreads, 0, s, g, nl, m, types_.data(), e, rc_sq_,
+               rho_.data(), fpp_.data(), G_.data(), wf_.data());
+        if (ntypes == 1) {
+          const size_t smem = sizeof(double) * 7 * static_cast<size_t>(W);
+          auto kern = k_fm_eam_pairs<Geo, L, true>;
+          TDMD_CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(smem)));
+          launch(kern, grid, kPairThreads, smem, s, g, nl, m, types_.data(), e, rc_sq_, G_.data(),
+                 wf_.data(), (nr - 1) - W, W, window_.data());
+          launch(k_fm_eam_window, ceil_div(7 * W, 32), 256, 0, s, window_.data(), grid, W,
+                 (nr - 1) - W, nr - 1, gphi, grho);
+        } else {
+          launch(k_fm_eam_pairs<Geo, L, false>, nblk, kThreads, 0, s, g, nl, m, types_.data(), e,
+                 rc_sq_, G_.data(), wf_.data(), 0, 0, nullptr);
+        }
       }
     });
-  });
+  };
+  if (mixed_)
+    passes(GeoQB{q_.data(), rep_.data(), scales_.data()},
+           GeoQB{recq_.data(), rep_.data(), scales_.data()});
+  else
+    passes(GeoD4B{pos4_.data(), rep_.data(), imgs_.data()},
+           GeoD4BF{rec_.data(), rep_.data(), imgs_.data()});
   TDMD_LAUNCH_CHECK();
-  launch(k_fm_sum, 1, kThreads, 0, s, part_.data(), nblk, 1, d_loss);
+  launch(k_fm_sum, 1, kThreads, 0, s, part_.data(), 1, d_loss, nullptr, 0, nullptr, nblk);
   TDMD_LAUNCH_CHECK();
 }
 

@@ -64,3 +64,42 @@ def test_fp64_pair_radius(cuda, r, wrapped):
     got = f.cpu().numpy()
     assert np.allclose(got[:, 0], [want_f, -want_f], rtol=1e-13, atol=1e-15)
     assert not got[:, 1:].any()
+
+
+# nr = 600: every interval inside the shared-memory window; 2000: the window's
+# lower edge at 1.8 A, below all pairs; 5001: at 3.72 A, so that the nearest
+# shell's pairs add to global memory and the others to the window
+@pytest.mark.parametrize("nr", [600, 2000, 5001])
+@pytest.mark.parametrize("ntypes", [1, 3])
+@pytest.mark.parametrize("nsnap", [1, 3])
+def test_eam_adjoint_window_edges(cuda, oracle, nr, ntypes, nsnap):
+    """EAM loss and gradient vs the FP64 oracle over the window's cases and a
+    grid of fewer blocks than SMs, atoms in random order: 1e-10 of the loss,
+    1e-9 of each spline's largest entry (sums of up to 1e4 terms of both
+    signs), as the other FP64 gradient tests."""
+    from tdmd_claude_b200 import Box, EamAlloy
+    from tdmd_claude_b200 import workloads as W
+    from tdmd_claude_b200.fitting import ForceMatch, eam_coeff_tensors, eam_table_meta
+    rng = np.random.default_rng(40 + nr + ntypes)
+    kw = {} if ntypes == 1 else dict(beta_f=(4.8, 5.0, 5.2), A_phi=(0.55, 0.60, 0.65),
+                                     E_F=(1.1, 1.2, 1.3))
+    t = W.analytic_eam(nr=nr, **kw)
+    eam = EamAlloy.from_tables(t.ntypes, t.nrho, t.drho, t.nr, t.dr, t.cutoff, t.F, t.rho, t.rphi)
+    lat = W.fcc_lattice(3, 3, 3, 3.615)
+    pos = np.stack([rng.permutation(lat + rng.normal(0, 0.1, lat.shape)) for _ in range(nsnap)])
+    L = 3 * 3.615
+    pos %= L
+    types = rng.integers(1, ntypes + 1, size=pos.shape[:2]).astype(np.int32)
+    tgt = rng.normal(0.0, 0.3, size=pos.shape)
+    fm = ForceMatch(pos, types, Box.make((0,) * 3, (L,) * 3), t.cutoff, "fp64")
+    fm.set_targets(tgt)
+    F, rho, phi = eam_coeff_tensors(eam)
+    loss = cuda.zeros(1, dtype=cuda.float64, device="cuda")
+    g = [cuda.empty_like(x) for x in (F, rho, phi)]
+    fm.eam(eam_table_meta(eam), F, rho, phi, loss, *g)
+    oe = oracle.OracleEam(t.ntypes, t.nrho, t.drho, t.nr, t.dr, t.cutoff, t.F, t.rho, t.rphi)
+    lo, *want = oe.fm_loss_grad(pos, types, (0,) * 3, (L,) * 3, tgt)
+    assert abs(loss.item() - lo) <= 1e-10 * lo
+    for got, ref in zip(g, want):
+        for sp in range(ref.shape[0]):
+            assert np.abs(got[sp].cpu().numpy() - ref[sp]).max() <= 1e-9 * np.abs(ref[sp]).max()
