@@ -323,6 +323,9 @@ struct tdmd_device_eam {
   EamDevTables tabs;
   DevArray<float> fp32;
   DevArray<double> fp64;
+  // energy/virial block partials: kept, because a pool allocation per call
+  // goes back to the driver at every synchronisation (0.4 to 5 ms to map again)
+  DevArray<double> part;
   // the reference's flat layout, for the ID-ordered energy mode
   RefEamTables ref;
 };
@@ -571,22 +574,22 @@ int32_t tdmd_device_eam_compute(tdmd_device_eam* de, const double* d_positions, 
     const int lpa = default_lpa(natoms);
     const int nblk = force_blocks(natoms, lpa);
     // Density records [0, nblk) and force records [nblk, 2*nblk).
-    Partials part(ev ? 2 * nblk : 0, s);
+    de->part.reserve(static_cast<size_t>(2 * nblk) * kEvStride);
     const int* types = de->tabs.ntypes > 1 ? d_types : nullptr;
     if (precision == TDMD_FP64) {
       de->fp64.reserve(static_cast<size_t>(natoms));
       const GeoAoS64 g{d_positions, img3(b)};
       launch_eam(g, nl, natoms, de->tabs.d64, types, de->fp64.data(), d_rho, d_fp,
-                 static_cast<double*>(d_forces), ev, part.p, lpa, s);
+                 static_cast<double*>(d_forces), ev, de->part.data(), lpa, s);
     } else {
       TDMD_REQUIRE(precision == TDMD_MIXED, "unknown precision");
       de->fp32.reserve(static_cast<size_t>(natoms));
       const GeoAoS32 g = make_geo_aos32(d_positions, b);
       launch_eam(g, nl, natoms, de->tabs.d32, types, de->fp32.data(), d_rho, d_fp,
-                 static_cast<float*>(d_forces), ev, part.p, lpa, s);
+                 static_cast<float*>(d_forces), ev, de->part.data(), lpa, s);
     }
     if (ev) {
-      launch(k_reduce_partials, 1, 256, 0, s, part.p, 2 * nblk, d_energy, d_virial);
+      launch(k_reduce_partials, 1, 256, 0, s, de->part.data(), 2 * nblk, d_energy, d_virial);
       TDMD_LAUNCH_CHECK();
     }
   });
