@@ -55,9 +55,9 @@ __global__ void __launch_bounds__(kThreads) k_morse_atom_pe(Geo g, NbrView nl, i
     const typename Geo::Own o = g.own(i);
     const long long row = nl.row(i);
     const int c = nl.count(i);
-    for (int base = U * sub; base < c; base += U * LPA) {
+    for (int base = first_slot<VEC, LPA, T, U>(sub); base < c; base += U * LPA) {
       int jj[U];
-      nbr_batch<VEC>(nl, row, base, c, jj);
+      nbr_batch<VEC, LPA, T>(nl, row, base, c, jj);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (jj[u] < 0) continue;
@@ -98,9 +98,9 @@ __global__ void __launch_bounds__(kThreads) k_eam_atom_pe(Geo g, NbrView nl, int
     const int ti = MULTI ? __ldg(types + i) - 1 : 0;
     const long long row = nl.row(i);
     const int c = nl.count(i);
-    for (int base = U * sub; base < c; base += U * LPA) {
+    for (int base = first_slot<VEC, LPA, T, U>(sub); base < c; base += U * LPA) {
       int jj[U];
-      nbr_batch<VEC>(nl, row, base, c, jj);
+      nbr_batch<VEC, LPA, T>(nl, row, base, c, jj);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (jj[u] < 0) continue;

@@ -94,27 +94,54 @@ __device__ __forceinline__ int2 ld_stream2(const int2* p) {
   return v;
 }
 
-// Indices base .. base+U-1 of a row (base < c, base a multiple of U), -1
-// past the count.  VEC: padded rows whose start is 16-byte aligned and whose
-// capacity is a multiple of 4 (vec_rows), so the vector read stays inside
-// the row: one int2 load for U = 2, one int4 load for U = 4.
-template <bool VEC, int U>
+__device__ __forceinline__ int ld_stream1(const int* p) {
+  int v;
+  asm volatile("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
+// The slots of a row that lane sub of an atom's LPA lanes takes in a sweep:
+// U consecutive ones in one vector load (kVectorRows), or every LPA-th one,
+// so that the lanes of an atom hold consecutive entries.  Consecutive entries
+// are mostly neighbors in memory (cell order), so a warp's record gathers
+// then touch fewer lines and meet less in a bank (counted on a 131k list, 8
+// lanes x 2: 13 lines and 25 bank cycles per 32 FP64 records instead of 17
+// and 28), and on dense rows the index loads coalesce.  FP64 and dense rows
+// gain (FP64 EAM 131k 5.74 -> 5.64 ms per 50 steps, Morse 256 815 -> 782 us
+// per 100, FP64 EAM evaluation of 40k atoms 69.8 -> 65.5 us); the 16-byte
+// mixed records do not (131k 3.86 -> 3.92 ms: more index loads than it
+// saves), so mixed padded rows keep the vector load, as do 1 to 4 lanes,
+// where a lane's own entries fill its sector.  Vector loads need padded rows
+// (VEC: 16-byte aligned, capacity a multiple of 4).
+template <bool VEC, int LPA, class T>
+constexpr bool kVectorRows = VEC && (LPA <= 4 || sizeof(T) == sizeof(float));
+
+// First sweep of lane sub; sweeps advance by U * LPA.
+template <bool VEC, int LPA, class T, int U>
+__device__ __forceinline__ int first_slot(int sub) {
+  return kVectorRows<VEC, LPA, T> ? U * sub : sub;
+}
+
+// Indices of the sweep at base < c, -1 past the count.
+template <bool VEC, int LPA, class T, int U>
 __device__ __forceinline__ void nbr_batch(const NbrView& nl, long long row, int base, int c,
                                           int (&j)[U]) {
   static_assert(U == 2 || U == 4, "neighbor batch: 2 or 4");
-  if constexpr (VEC && U == 2) {
+  if constexpr (kVectorRows<VEC, LPA, T> && U == 2) {
     const int2 v = ld_stream2(reinterpret_cast<const int2*>(nl.nbr + row + base));
     j[0] = v.x;
     j[1] = base + 1 < c ? v.y : -1;
-  } else if constexpr (VEC) {
+  } else if constexpr (kVectorRows<VEC, LPA, T>) {
     const int4 v = ld_stream(reinterpret_cast<const int4*>(nl.nbr + row + base));
     j[0] = v.x;
     j[1] = base + 1 < c ? v.y : -1;
     j[2] = base + 2 < c ? v.z : -1;
     j[3] = base + 3 < c ? v.w : -1;
   } else {
+    const int* const r = nl.nbr + row + base;
 #pragma unroll
-    for (int u = 0; u < U; ++u) j[u] = base + u < c ? __ldg(nl.nbr + row + base + u) : -1;
+    for (int u = 0; u < U; ++u)
+      j[u] = base + u * LPA < c ? (VEC ? ld_stream1(r + u * LPA) : __ldg(r + u * LPA)) : -1;
   }
 }
 
@@ -565,9 +592,9 @@ __global__ void __launch_bounds__(256) k_morse(Geo g, NbrView nl, int n,
     const long long row = nl.row(i);
     const int c = nl.count(i);
     const T two_d_alpha = T(2) * mp.d * mp.alpha;
-    for (int base = U * sub; base < c; base += U * LPA) {
+    for (int base = first_slot<VEC, LPA, T, U>(sub); base < c; base += U * LPA) {
       int jj[U];
-      nbr_batch<VEC>(nl, row, base, c, jj);
+      nbr_batch<VEC, LPA, T>(nl, row, base, c, jj);
       typename Geo::Pair pr[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -809,9 +836,9 @@ __global__ void __launch_bounds__(256) k_eam_density(Geo g, NbrView nl, int n,
     o = g.own(i);
     const long long row = nl.row(i);
     const int c = nl.count(i);
-    for (int base = U * sub; base < c; base += U * LPA) {
+    for (int base = first_slot<VEC, LPA, T, U>(sub); base < c; base += U * LPA) {
       int jj[U];
-      nbr_batch<VEC>(nl, row, base, c, jj);
+      nbr_batch<VEC, LPA, T>(nl, row, base, c, jj);
       typename Geo::Pair pr[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -956,9 +983,9 @@ __global__ void __launch_bounds__(256) k_eam_force(Geo g, NbrView nl, int n,
       fpi = packed ? __int_as_float(g.record(o).w & ~tmask) : static_cast<T>(__ldg(fp + i));
     else
       fpi = static_cast<T>(__ldg(fp + i));
-    for (int base = U * sub; base < c; base += U * LPA) {
+    for (int base = first_slot<VEC, LPA, T, U>(sub); base < c; base += U * LPA) {
       int jj[U];
-      nbr_batch<VEC>(nl, row, base, c, jj);
+      nbr_batch<VEC, LPA, T>(nl, row, base, c, jj);
       typename Geo::Pair pr[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {

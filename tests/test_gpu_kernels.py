@@ -103,3 +103,30 @@ def test_eam_adjoint_window_edges(cuda, oracle, nr, ntypes, nsnap):
     for got, ref in zip(g, want):
         for sp in range(ref.shape[0]):
             assert np.abs(got[sp].cpu().numpy() - ref[sp]).max() <= 1e-9 * np.abs(ref[sp]).max()
+
+
+# rows shorter than a sweep, one past whole sweeps, and longer; every lane count
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8, 16, 32])
+@pytest.mark.parametrize("batch", [2, 4])
+def test_lane_slots_cover_every_row(cuda, oracle, precision, lanes, batch):
+    """A gas whose rows hold 0 to ~70 entries: every slot of every row is
+    taken once whatever the lanes and sweep (forces vs the oracle to 1e-10 of
+    their RMS in FP64, 1e-5 in mixed, the library's bounds)."""
+    from tdmd_claude_b200 import Box, FastPipelineScheduler, MorseParams, make_config
+    rng = np.random.default_rng(6)
+    pos = np.concatenate([rng.uniform(0, 30.0, (150, 3)), rng.uniform(10.0, 18.0, (65, 3))])
+    n, morse = len(pos), (0.05, 1.0, 3.0, 5.0)
+    s = FastPipelineScheduler(Box.make((0,) * 3, (30.0,) * 3), n, MorseParams.make(*morse),
+                              make_config(r_skin=0.4, precision=precision, lanes_per_atom=lanes,
+                                          nbr_batch=batch))
+    masses = np.array([1.0, 63.546])
+    s.upload(pos, np.zeros((n, 3)), None, np.ones(n, np.int32), None, masses)
+    s.run_until(0)
+    cnt = s.neighbor_list()[0]
+    assert cnt.min() == 0 and cnt.max() > 32
+    want = oracle.md_run(pos, np.zeros((n, 3)), np.ones(n, np.int32), masses, (0,) * 3,
+                         (30.0,) * 3, 0.001, 0.4, 10, [0], morse=morse)["forces"]
+    d = s.download().forces - want
+    rms = np.sqrt((want ** 2).mean())
+    assert np.sqrt((d ** 2).mean()) <= (1e-10 if precision == "fp64" else 1e-5) * rms
