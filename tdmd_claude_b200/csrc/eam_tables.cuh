@@ -54,6 +54,7 @@ struct EamDevTables {
   DevArray<double4> ftab;
   DevArray<double4> deriv4;  // one type, FP64: derivative rows split in two
   DevArray<double2> deriv2;
+  DevArray<double> deriva;
   EamDev<double> d64{};
   EamDev<float> d32{};
   int ntypes = 0;

@@ -349,6 +349,7 @@ struct GeoD4F {
 
 struct GeoAoS64 {  // FP64, reference Vec3D AoS
   using T = double;
+  static constexpr bool kD4Out = true;
   static constexpr bool kRecords = false;
   using Own = double3;
   using Pair = PairD;
@@ -675,10 +676,11 @@ struct EamDev {
   // F' below 2^(tbits-23)), so the force pass gathers no type; 0 = types are
   // gathered (one type, or more than 16).
   int tbits;
-  // One type, FP64, forces only: the six derivative coefficients of a bin as
-  // (rho' b, 2c, 3d, phi' b) and (phi' 2c, 3d).
+  // One type, FP64: the six derivative coefficients of a bin as
+  // (rho' b, 2c, 3d, phi' b) and (phi' 2c, 3d), and phi's a for the energy.
   const double4* d4 = nullptr;
   const double2* d2 = nullptr;
+  const double* da = nullptr;
 };
 
 __device__ __forceinline__ int phi_slot(int ti, int tj, int nt) {
@@ -1011,8 +1013,9 @@ __global__ void __launch_bounds__(256) k_eam_force(Geo g, NbrView nl, int n,
           typename V4<T>::type cphi, crho;
           if constexpr (!MULTI && sizeof(T) == sizeof(float)) {
             ld_rows2(rowp, crho, cphi);  // single type: S = 2, slots rho', phi'
-          } else if constexpr (!MULTI && EV == 0) {
+          } else if constexpr (!MULTI) {
             ld_derivs(e, idx, crho, cphi);
+            if (EV) cphi.w = __ldg(e.da + idx);
           } else {
             cphi = ldv4<T>(rowp + (MULTI ? phi_slot(ti, tj, e.ntypes) : 1));
             crho = ldv4<T>(rowp + tj);
@@ -1070,6 +1073,11 @@ __global__ void __launch_bounds__(256) k_eam_force(Geo g, NbrView nl, int n,
 // ADDS them to energy[0] / virial[0..5] (either may be null).
 __global__ void k_reduce_partials(const double* __restrict__ partials, int nblk,
                                   double* __restrict__ energy, double* __restrict__ virial);
+
+// Threads of that one block: the records are a serial chain of loads per
+// thread, so more than 512 records take 1024 threads (2530 records: 8.5 us
+// with 256).
+inline int reduce_threads(int nblk) { return nblk > 512 ? 1024 : 256; }
 
 int force_blocks(long long n, int lpa);
 
