@@ -130,3 +130,22 @@ def test_lane_slots_cover_every_row(cuda, oracle, precision, lanes, batch):
     d = s.download().forces - want
     rms = np.sqrt((want ** 2).mean())
     assert np.sqrt((d ** 2).mean()) <= (1e-10 if precision == "fp64" else 1e-5) * rms
+
+
+def test_neighbor_list_handle_reused(cuda, oracle):
+    """One handle over changing inputs: the first build (two sweeps), the same
+    atoms again, a squeezed system whose rows overflow the kept capacity, a
+    dilute one, another atom count: rows bit-exact to the oracle each time."""
+    from tdmd_claude_b200 import Box, DeviceNeighborList
+    rng = np.random.default_rng(8)
+    a = rng.uniform(0, 30.0, (1500, 3))
+    squeezed = 9.0 + a * 0.4
+    cases = [a, a, a + 0.01, squeezed, squeezed, a, a[:777], a[:1], a]
+    nl = DeviceNeighborList()
+    for k, p in enumerate(cases):
+        p = np.ascontiguousarray(p % 30.0)
+        nl.build(_dev(cuda, p), len(p), Box.make((0,) * 3, (30.0,) * 3), 4.0, 0.3)
+        c, o, nb = nl.host_csr()
+        ec, eo, enb = oracle.neighbor_list(p, (0,) * 3, (30.0,) * 3, 4.0, 0.3, half=False)
+        assert np.array_equal(c, ec) and np.array_equal(o, eo) and np.array_equal(nb, enb), k
+        assert nl.max_neighbors() == int(ec.max()) and nl.total_pairs() == enb.size
