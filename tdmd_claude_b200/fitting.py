@@ -13,6 +13,7 @@ src/potentials/eam_alloy.cpp:196-295.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import time
 
 import numpy as np
@@ -178,7 +179,10 @@ class ShardedForceMatch:
             self.local.close()
 
 
+@functools.lru_cache(maxsize=None)
 def _autograd():
+    """The autograd classes, made on first use (importing this module does not
+    import torch) and once: making the two classes took 41 us of every loss call."""
     import torch
 
     class MorseLoss(torch.autograd.Function):
