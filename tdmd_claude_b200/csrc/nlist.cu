@@ -171,6 +171,13 @@ __global__ void k_sort_cells(const int* __restrict__ cell_start, const int* __re
 // the center cell.
 // --------------------------------------------------------------------------
 constexpr int kRowThreads = 128;
+// One system of few cells (at most two per SM) gets CTAs of 512 threads: with
+// the chip idle, the time is one cell's serial chain -- staging, then the rows
+// a warp takes in turn -- and more warps shorten it.  Above that the smaller
+// CTAs fill the SMs better (131k, 9 261 cells: 64 and 128 threads compared).
+// 256 atoms, 27 cells: 808 -> 758 us per 100 steps; 2 767 atoms, 140 cells:
+// 1.31 -> 1.22 ms.
+constexpr int kRowThreadsFew = 512;
 constexpr int kStageCap = 1536;  // staged candidate records (24 KiB)
 constexpr int kSlabMax = 128;    // center atoms handled as warp slabs
 constexpr int kIdxCap = 512;     // kept candidates per warp slab
@@ -195,10 +202,11 @@ __device__ __noinline__ bool exact_within(Load pos, int i, int j, double rl2, do
 }
 
 // Shared memory of one row-building CTA.
+template <int RT>
 struct RowSmem {
   int s_start[27], s_pre[28];
-  int s_max[kRowThreads / 32];
-  int s_wcnt[kRowThreads / 32];  // kept candidates per warp (staging chunk)
+  int s_max[RT / 32];
+  int s_wcnt[RT / 32];  // kept candidates per warp (staging chunk)
   float s_bb[6];                 // center cell's bounding box: min xyz, max xyz
   int s_c0;                      // staged index of the center cell's first atom
 };
@@ -217,9 +225,9 @@ __device__ __forceinline__ float r2_rn(float dx, float dy, float dz) {
 
 // Rows of the atoms of cell c of box b's grid; cell_start / cell_count index
 // that grid's cells, cell_atoms and the atom indices are global.
-template <class Load, bool WRAP, bool WRITE, bool SLAB>
+template <int RT, class Load, bool WRAP, bool WRITE, bool SLAB>
 __device__ __forceinline__ void build_cell_rows(
-    RowSmem& sm, float4* stage, int stage_cap, SlabSmem* ss, Load pos, const DevBox& b, int c,
+    RowSmem<RT>& sm, float4* stage, int stage_cap, SlabSmem* ss, Load pos, const DevBox& b, int c,
     const int* __restrict__ cell_start,
     const int* __restrict__ cell_count, const int* __restrict__ cell_atoms, double rl2,
     float lo_f, float hi_f, int* __restrict__ nbr, const int* __restrict__ row_off, int cap,
@@ -348,12 +356,12 @@ __device__ __forceinline__ void build_cell_rows(
     // center atoms ranked by x and cut into one contiguous slab per warp;
     // each warp keeps, in candidate order, the candidates within the band
     // of its slab's bounding box (an index list), and sweeps only those.
-    for (int k = threadIdx.x; k < total; k += kRowThreads) stage[k] = record(k);
+    for (int k = threadIdx.x; k < total; k += RT) stage[k] = record(k);
     if (threadIdx.x == 0) stage[total] = sentinel;
     __syncthreads();
     // (a far record's NaN x ranks as +inf, so the ranks stay a permutation)
     auto xkey = [](float x) { return x == x ? x : INFINITY; };
-    for (int t = threadIdx.x; t < ncen; t += kRowThreads) {
+    for (int t = threadIdx.x; t < ncen; t += RT) {
       const float xt = xkey(stage[c0 + t].x);
       int rank = 0;
       for (int u = 0; u < ncen; ++u) {
@@ -363,7 +371,7 @@ __device__ __forceinline__ void build_cell_rows(
       ss->s_order[rank] = static_cast<short>(t);
     }
     __syncthreads();
-    constexpr int kWarps = kRowThreads / 32;
+    constexpr int kWarps = RT / 32;
     const int rlo = warp * ncen / kWarps, rhi = (warp + 1) * ncen / kWarps;
     if (rlo < rhi) {
       float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -425,7 +433,7 @@ __device__ __forceinline__ void build_cell_rows(
     int kept = total;  // staged candidates (after pruning)
     if (staged) {
       if (WRAP) {
-        for (int k = threadIdx.x; k < total; k += kRowThreads) stage[k] = record(k);
+        for (int k = threadIdx.x; k < total; k += RT) stage[k] = record(k);
       } else {
         if (warp == 0) {
           float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -458,7 +466,7 @@ __device__ __forceinline__ void build_cell_rows(
         const float bx0 = sm.s_bb[0], by0 = sm.s_bb[1], bz0 = sm.s_bb[2];
         const float bx1 = sm.s_bb[3], by1 = sm.s_bb[4], bz1 = sm.s_bb[5];
         kept = 0;
-        for (int k0 = 0; k0 < total; k0 += kRowThreads) {
+        for (int k0 = 0; k0 < total; k0 += RT) {
           const int k = k0 + threadIdx.x;
           float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
           bool keep = false;
@@ -474,7 +482,7 @@ __device__ __forceinline__ void build_cell_rows(
           __syncthreads();
           int off = kept, tot = kept;
 #pragma unroll
-          for (int w = 0; w < kRowThreads / 32; ++w) {
+          for (int w = 0; w < RT / 32; ++w) {
             const int cw = sm.s_wcnt[w];
             off += w < warp ? cw : 0;
             tot += cw;
@@ -486,7 +494,7 @@ __device__ __forceinline__ void build_cell_rows(
           __syncthreads();
         }
       }
-      for (int k = kept + threadIdx.x; k < ((kept + 31) & ~31); k += kRowThreads)
+      for (int k = kept + threadIdx.x; k < ((kept + 31) & ~31); k += RT)
         stage[k] = sentinel;
     }
     __syncthreads();
@@ -495,11 +503,11 @@ __device__ __forceinline__ void build_cell_rows(
     const int cbase = (staged && !WRAP && ncen > 0) ? sm.s_c0 : c0;
     // staged records (the hot path) or records rebuilt on the fly
     if (staged) {
-      for (int a = warp; a < ncen; a += kRowThreads / 32)
+      for (int a = warp; a < ncen; a += RT / 32)
         row(stage[cbase + a], cbase + a, [&](int k) { return stage[k]; }, ncand,
             std::true_type{});
     } else {
-      for (int a = warp; a < ncen; a += kRowThreads / 32)
+      for (int a = warp; a < ncen; a += RT / 32)
         row(record(cbase + a), cbase + a, record, ncand, std::false_type{});
     }
   }
@@ -512,7 +520,7 @@ __device__ __forceinline__ void build_cell_rows(
     __syncthreads();
     if (threadIdx.x == 0) {
       int m = 0;
-      for (int w = 0; w < kRowThreads / 32; ++w) m = s_max[w] > m ? s_max[w] : m;
+      for (int w = 0; w < RT / 32; ++w) m = s_max[w] > m ? s_max[w] : m;
       const bool overflow = WRITE && !row_off && m > cap;
       if (overflow) atomicOr(&status[0], 1);
       if (overflow || !WRITE || report_max) atomicMax(&status[1], m);
@@ -520,8 +528,8 @@ __device__ __forceinline__ void build_cell_rows(
   }
 }
 
-template <class Load, bool WRAP, bool WRITE>
-__global__ void __launch_bounds__(kRowThreads) k_build_cells(
+template <int RT, class Load, bool WRAP, bool WRITE>
+__global__ void __launch_bounds__(RT) k_build_cells(
     Load pos, DevBox b, const int* __restrict__ cell_start, const int* __restrict__ cell_count,
     const int* __restrict__ cell_atoms, double rl2, float lo_f, float hi_f, int* __restrict__ nbr,
     const int* __restrict__ row_off, int cap, int* __restrict__ counts,
@@ -530,8 +538,8 @@ __global__ void __launch_bounds__(kRowThreads) k_build_cells(
   // The stage is dynamic shared memory of stage_cap records (sized by the
   // launch from the mean cell occupancy, so that more CTAs fit on an SM).
   extern __shared__ float4 stage[];
-  __shared__ RowSmem sm;
-  build_cell_rows<Load, WRAP, WRITE, false>(sm, stage, stage_cap, nullptr, pos, b, blockIdx.x,
+  __shared__ RowSmem<RT> sm;
+  build_cell_rows<RT, Load, WRAP, WRITE, false>(sm, stage, stage_cap, nullptr, pos, b, blockIdx.x,
                                             cell_start, cell_count, cell_atoms, rl2, lo_f, hi_f,
                                             nbr, row_off, cap, counts, status, report_max != 0);
 }
@@ -547,19 +555,19 @@ __global__ void __launch_bounds__(kRowThreads) k_build_cells_batch(
     int* __restrict__ counts, int* __restrict__ status) {
   dependent_launch_prologue();
   __shared__ float4 stage[kStageCap];
-  __shared__ RowSmem sm;
+  __shared__ RowSmem<kRowThreads> sm;
   __shared__ SlabSmem ss;
   __shared__ RepDesc d;
   const int gc = blockIdx.x;
   if (threadIdx.x == 0) d = reps[__ldg(cell_rep + gc)];
   __syncthreads();
   if (d.wrap)
-    build_cell_rows<LoadD4, true, WRITE, true>(sm, stage, kStageCap, &ss, pos, d.box, gc - d.cell0,
+    build_cell_rows<kRowThreads, LoadD4, true, WRITE, true>(sm, stage, kStageCap, &ss, pos, d.box, gc - d.cell0,
                                                cell_start + d.cell0, cell_count + d.cell0,
                                                cell_atoms, rl2, d.lo_f, d.hi_f, nbr, nullptr,
                                                cap, counts, status, false);
   else
-    build_cell_rows<LoadD4, false, WRITE, true>(sm, stage, kStageCap, &ss, pos, d.box,
+    build_cell_rows<kRowThreads, LoadD4, false, WRITE, true>(sm, stage, kStageCap, &ss, pos, d.box,
                                                 gc - d.cell0,
                                                 cell_start + d.cell0, cell_count + d.cell0,
                                                 cell_atoms, rl2, d.lo_f, d.hi_f, nbr, nullptr,
@@ -724,16 +732,24 @@ void build_neighbor_rows(const CellListDev& cl, const void* d_pos, PosLayout lay
   row_filter_band(box, r_list_sq, &lo_f, &hi_f, &wrap);
   const int scap = stage_capacity(max_cell);
   const size_t smem = sizeof(float4) * static_cast<size_t>(scap);
-  auto go = [&](auto load, auto wrap_tag) {
+  auto go_threads = [&](auto load, auto wrap_tag, auto threads_tag) {
     constexpr bool W = decltype(wrap_tag)::value;
+    constexpr int RT = decltype(threads_tag)::value;
     if (nbr)
-      launch(k_build_cells<decltype(load), W, true>, cl.ncells, kRowThreads, smem, stream, load,
+      launch(k_build_cells<RT, decltype(load), W, true>, cl.ncells, RT, smem, stream, load,
              box, cl.cell_start.data(), cl.cell_count.data(), cl.cell_atoms.data(), r_list_sq, lo_f,
              hi_f, nbr, row_off, cap, counts, status, scap, report_max ? 1 : 0);
     else
-      launch(k_build_cells<decltype(load), W, false>, cl.ncells, kRowThreads, smem, stream, load,
+      launch(k_build_cells<RT, decltype(load), W, false>, cl.ncells, RT, smem, stream, load,
              box, cl.cell_start.data(), cl.cell_count.data(), cl.cell_atoms.data(), r_list_sq, lo_f,
              hi_f, nullptr, row_off, cap, counts, status, scap, 0);
+  };
+  const bool few = cl.ncells <= 2 * sm_count();
+  auto go = [&](auto load, auto wrap_tag) {
+    if (few)
+      go_threads(load, wrap_tag, std::integral_constant<int, kRowThreadsFew>{});
+    else
+      go_threads(load, wrap_tag, std::integral_constant<int, kRowThreads>{});
   };
   if (layout == PosLayout::AoS3) {
     const LoadAoS3 ld{static_cast<const double*>(d_pos)};

@@ -149,3 +149,22 @@ def test_neighbor_list_handle_reused(cuda, oracle):
         ec, eo, enb = oracle.neighbor_list(p, (0,) * 3, (30.0,) * 3, 4.0, 0.3, half=False)
         assert np.array_equal(c, ec) and np.array_equal(o, eo) and np.array_equal(nb, enb), k
         assert nl.max_neighbors() == int(ec.max()) and nl.total_pairs() == enb.size
+
+
+# two cells per SM are 296 on a B200: 270 and 540 cells with 3-cell axes, 294
+# and 300 without
+@pytest.mark.parametrize("nc", [(3, 3, 30), (3, 3, 60), (7, 7, 6), (5, 6, 10)])
+def test_row_build_block_sizes(cuda, oracle, nc):
+    """The list on both sides of the few-cells rule, with and without 3-cell
+    axes, a dense corner included: bit-exact to the oracle."""
+    from tdmd_claude_b200 import Box, DeviceNeighborList
+    rng = np.random.default_rng(9)
+    r, hi = 4.4, np.array(nc) * 4.5
+    p = np.concatenate([rng.uniform(0, 1, (10 * int(np.prod(nc)), 3)) * hi,
+                        rng.uniform(0, 1, (300, 3)) * 6.0])
+    nl = DeviceNeighborList()
+    nl.build(_dev(cuda, p), len(p), Box.make((0,) * 3, hi), r - 0.3, 0.3)
+    got = nl.host_csr()
+    want = oracle.neighbor_list(p, (0,) * 3, tuple(hi), r - 0.3, 0.3, half=False)
+    for g, w in zip(got, want):
+        assert np.array_equal(g, w)
