@@ -89,6 +89,9 @@ enum class PosLayout { AoS3, D4 };
 void build_cell_list(CellListDev& cl, const void* d_pos, PosLayout layout, long long n,
                      const DevBox& box, cudaStream_t stream, const int* key = nullptr);
 
+// Kernels that build_cell_list launches for n atoms in ncells cells.
+int cell_list_launches(long long n, long long ncells);
+
 // Neighbor list build over a built cell list.
 //   row_off == nullptr: padded rows, entry k of atom i at nbr[i*cap + k];
 //                       status[0] |= 1 when some atom has more than cap.

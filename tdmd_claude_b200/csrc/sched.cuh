@@ -157,8 +157,7 @@ class Scheduler {
   void prof_begin(int cat);
   void prof_end(int cat);
   void prof_collect();
-  // bin + scan + scatter + sort
-  int cell_list_kernels() const { return 3 + device_scan_launches(cl_.ncells); }
+  int cell_list_kernels() const { return cell_list_launches(n_, cl_.ncells); }
   void reorder_by_cell(cudaEvent_t side_done = nullptr);
   // Keyed cell list of the current positions; returns the kernels launched.
   int build_cells();

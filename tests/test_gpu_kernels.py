@@ -168,3 +168,23 @@ def test_row_build_block_sizes(cuda, oracle, nc):
     want = oracle.neighbor_list(p, (0,) * 3, tuple(hi), r - 0.3, 0.3, half=False)
     for g, w in zip(got, want):
         assert np.array_equal(g, w)
+
+
+# the one-block rule's two limits (4096 atoms, 512 cells) and both sides of each
+@pytest.mark.parametrize("n,nc", [(1, (3, 3, 3)), (31, (3, 4, 5)), (4096, (8, 8, 8)),
+                                  (4097, (8, 8, 8)), (4000, (9, 8, 8)), (4096, (3, 3, 3))])
+def test_cell_list_one_block(cuda, oracle, n, nc):
+    """Cell lists bit-exact around the one-block limits, with cells above 32
+    and above 128 members (27 cells of ~150 atoms)."""
+    from tdmd_claude_b200 import Box, DeviceCellList
+    rng = np.random.default_rng(n)
+    hi = np.array(nc) * 5.0 + 0.1
+    p = rng.uniform(-0.01, 1.01, (n, 3)) * hi  # some atoms outside: clamped
+    cl = DeviceCellList()
+    cl.build(_dev(cuda, p), n, Box.make((0,) * 3, hi), 5.0)
+    got = cl.arrays()
+    want = oracle.cell_list(p, (0,) * 3, tuple(hi), 5.0)
+    assert tuple(got[0]) == nc
+    enc, ecc, eco, eca, eac = want
+    for g, w in zip(got, (enc, eca, eco, ecc, eac)):
+        assert np.array_equal(g, w)
