@@ -183,9 +183,10 @@ __global__ void k_unpack_batch(const double4* __restrict__ pos4, int n, double* 
 // Kick (half or full dt) + drift + single-image wrap in the atom's replica
 // box + fixed-point refresh; fused_kick_drift_kernel,
 // device_velocity_verlet.cu:88-130, per replica.
+// pos4_out may be pos4.
 template <class F, bool FULL>
 __global__ void __launch_bounds__(kThreads) k_kick_drift_batch(
-    double4* __restrict__ pos4, int4* __restrict__ q, double* __restrict__ v,
+    const double4* pos4, double4* pos4_out, int4* __restrict__ q, double* __restrict__ v,
     const F* __restrict__ f, const int* __restrict__ types, const int* __restrict__ rep,
     const RepDesc* __restrict__ reps, const double* __restrict__ inv_mm, int n, double dt) {
   dependent_launch_prologue();
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(kThreads) k_kick_drift_batch(
   v[3ll * i] = vx;
   v[3ll * i + 1] = vy;
   v[3ll * i + 2] = vz;
-  pos4[i] = p;
+  pos4_out[i] = p;
   if (q)
     q[i] = make_int4(encode_q(p.x, b.qlo[0], b.qinv[0]), encode_q(p.y, b.qlo[1], b.qinv[1]),
                      encode_q(p.z, b.qlo[2], b.qinv[2]), t);
@@ -231,6 +232,7 @@ struct BatchStep {
   bool first, rebuild;
   bool kd_fused;   // kick + drift done by the previous step's force pass
   bool fuse_next;  // this force pass also kicks and drifts for the next step
+  bool to_alt;     // the kick + drift launch writes to the second position buffers
   bool log_e;      // window end of a logged window: the force pass also writes
                    // per-atom energies, reduced per replica after the half kick
 };
@@ -280,7 +282,7 @@ class Batch {
   static constexpr int kPassDensity = 1, kPassForce = 2, kPassBoth = 3;
   void force(bool kd = false, bool pe_atom = false, int parts = kPassBoth);
   void rep_energy();
-  void kick_drift(bool full);
+  void kick_drift(bool full, bool to_alt);
   void half_kick();
   void enqueue_step(const BatchStep& st);
   void run_segment(const std::vector<BatchStep>& seg, bool finalize, bool prologue);
@@ -328,6 +330,13 @@ class Batch {
   DevArray<int> rep_;
   DevArray<double4> pos4_;
   DevArray<int4> q_;
+  // second position buffers of the fused Morse passes, and whether they hold
+  // the positions now (inside a window only)
+  DevArray<double4> pos4_alt_;
+  DevArray<int4> q_alt_;
+  bool in_alt_ = false;
+  double4* pos4() const { return in_alt_ ? pos4_alt_.data() : pos4_.data(); }
+  int4* q() const { return in_alt_ ? q_alt_.data() : q_.data(); }
   DevArray<double> vel_;
   DevArray<float> f32_;
   DevArray<double> f64_;
@@ -558,8 +567,8 @@ void Batch::grow_capacity(int max_count) {
 
 void Batch::rebuild(int* status) {
   cudaStream_t s = stream_;
-  build_cell_list_batch(cl_, pos4_.data(), rep_.data(), reps_.data(), n_, ncells_, s);
-  build_neighbor_rows_batch(cl_, pos4_.data(), reps_.data(), cell_rep_.data(), rl2_,
+  build_cell_list_batch(cl_, pos4(), rep_.data(), reps_.data(), n_, ncells_, s);
+  build_neighbor_rows_batch(cl_, pos4(), reps_.data(), cell_rep_.data(), rl2_,
                             nbr_.data(), cap_, cnt_.data(), status, s);
   launches_ += 4 + device_scan_launches(ncells_);
   ++rebuilds_;
@@ -571,8 +580,7 @@ void Batch::force(bool kd, bool pea, int parts) {
   const int n = static_cast<int>(n_);
   const Tune td{lpa_d_, nu_d_}, tf{lpa_, nu_};
   const bool dens = parts & kPassDensity, pair = parts & kPassForce;
-  TDMD_REQUIRE(!kd || eam_, "fused kick-drift needs the EAM batch");
-  if (eam_) {
+    if (eam_) {
     // Density + embedding, then forces, over all replicas at once (the
     // single scheduler's passes on the batched geometries).
     const int* types = eam_->ntypes > 1 ? types_.data() : nullptr;
@@ -612,38 +620,48 @@ void Batch::force(bool kd, bool pea, int parts) {
     launches_ += (dens ? 1 : 0) + (pair ? 1 : 0);
     return;
   }
+  // kd: the next step's kick + drift in the same pass, into the other buffers
+  const KickDrift kdr{pos4(),         nullptr,      vel_.data(),
+                      types_.data(),  inv_mm_.data(), cfg_.dt,
+                      nullptr,        DevBox{},     rep_.data(),
+                      reps_.data(),   in_alt_ ? pos4_.data() : pos4_alt_.data(),
+                      in_alt_ ? q_.data() : q_alt_.data()};
   if (mixed_) {
-    const GeoQB g{q_.data(), rep_.data(), scales_.data()};
-    launch_morse(g, nl, n, m32_, f32_.data(), pea, nullptr, tf, s,
-                 pea ? pe_atom_.data() : nullptr);
+    const GeoQB g{q(), rep_.data(), scales_.data()};
+    launch_morse<true>(g, nl, n, m32_, f32_.data(), pea, nullptr, tf, s,
+                       pea ? pe_atom_.data() : nullptr, kd ? &kdr : nullptr);
   } else {
-    const GeoD4B g{pos4_.data(), rep_.data(), imgs_.data()};
-    launch_morse(g, nl, n, m64_, f64_.data(), pea, nullptr, tf, s,
-                 pea ? pe_atom_.data() : nullptr);
+    const GeoD4B g{pos4(), rep_.data(), imgs_.data()};
+    launch_morse<true>(g, nl, n, m64_, f64_.data(), pea, nullptr, tf, s,
+                       pea ? pe_atom_.data() : nullptr, kd ? &kdr : nullptr);
   }
+  if (kd) in_alt_ = !in_alt_;
   ++launches_;
 }
 
-void Batch::kick_drift(bool full) {
+void Batch::kick_drift(bool full, bool to_alt) {
   cudaStream_t s = stream_;
+  double4* const from = pos4();
+  if (to_alt) in_alt_ = !in_alt_;
+  double4* const to = pos4();
   const int n = static_cast<int>(n_);
   const int nb = ceil_div(n_, kThreads);
   if (mixed_) {
     if (full)
-      launch(k_kick_drift_batch<float, true>, nb, kThreads, 0, s, pos4_.data(), q_.data(),
+      launch(k_kick_drift_batch<float, true>, nb, kThreads, 0, s, from, to, q(),
              vel_.data(), f32_.data(), types_.data(), rep_.data(), reps_.data(), inv_mm_.data(), n,
              cfg_.dt);
     else
-      launch(k_kick_drift_batch<float, false>, nb, kThreads, 0, s, pos4_.data(), q_.data(),
+      launch(k_kick_drift_batch<float, false>, nb, kThreads, 0, s, from, to, q(),
              vel_.data(), f32_.data(), types_.data(), rep_.data(), reps_.data(), inv_mm_.data(), n,
              cfg_.dt);
   } else {
     if (full)
-      launch(k_kick_drift_batch<double, true>, nb, kThreads, 0, s, pos4_.data(), nullptr,
+      launch(k_kick_drift_batch<double, true>, nb, kThreads, 0, s, from, to, nullptr,
              vel_.data(), f64_.data(), types_.data(), rep_.data(), reps_.data(), inv_mm_.data(), n,
              cfg_.dt);
     else
-      launch(k_kick_drift_batch<double, false>, nb, kThreads, 0, s, pos4_.data(), nullptr,
+      launch(k_kick_drift_batch<double, false>, nb, kThreads, 0, s, from, to, nullptr,
              vel_.data(), f64_.data(), types_.data(), rep_.data(), reps_.data(), inv_mm_.data(), n,
              cfg_.dt);
   }
@@ -669,7 +687,7 @@ void Batch::half_kick() {
 // kick-drift (half kick on the first step of a window), rebuild when due,
 // forces; the window closes with a half kick.
 void Batch::enqueue_step(const BatchStep& st) {
-  if (!st.kd_fused) kick_drift(!st.first);
+  if (!st.kd_fused) kick_drift(!st.first, st.to_alt);
   if (st.rebuild) rebuild(status_.data());
   force(st.fuse_next, st.log_e);
 }
@@ -696,9 +714,12 @@ void Batch::run_segment(const std::vector<BatchStep>& seg, bool finalize, bool p
   key.reserve(seg.size() + 2);
   for (const auto& st : seg)
     key.push_back((st.first ? 1 : 0) | (st.rebuild ? 2 : 0) | (st.kd_fused ? 4 : 0) |
-                  (st.fuse_next ? 8 : 0) | (st.log_e ? 16 : 0));
+                  (st.fuse_next ? 8 : 0) | (st.log_e ? 16 : 0) | (st.to_alt ? 32 : 0));
   key.push_back(finalize ? 1 : 0);
   key.push_back(prologue ? 1 : 0);
+  key.push_back(in_alt_ ? 1 : 0);
+  bool end_in_alt = in_alt_;  // where the segment leaves the positions
+  for (const auto& st : seg) end_in_alt = end_in_alt != (st.to_alt != (st.fuse_next && !eam_));
   const long long l0 = launches_;
   // the window's closing half kick, then (logged windows) the per-replica
   // energies of the integer-time state
@@ -724,12 +745,14 @@ void Batch::run_segment(const std::vector<BatchStep>& seg, bool finalize, bool p
       graph_lru_.pop_back();
     }
     cudaGraph_t g = nullptr;
+    const bool start_in_alt = in_alt_;
     TDMD_CU(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     try {
       if (prologue) enqueue_prologue();
       for (const auto& st : seg) enqueue_step(st);
       close();
     } catch (...) {
+      in_alt_ = start_in_alt;
       cudaStreamEndCapture(stream_, &g);
       if (g) cudaGraphDestroy(g);
       throw;
@@ -748,6 +771,7 @@ void Batch::run_segment(const std::vector<BatchStep>& seg, bool finalize, bool p
     graph_lru_.push_front(key);
   }
   TDMD_CU(cudaGraphLaunch(it->second.first, stream_));
+  in_alt_ = end_in_alt;
   launches_ += it->second.second;
   ++graph_launches_;
 }
@@ -854,7 +878,16 @@ void Batch::run_until(int target) {
   snap_pos4_.reserve(n);
   snap_vel_.reserve(3 * n);
   if (mixed_) snap_q_.reserve(n);
+  // Morse graph windows: the force passes carry the next step's kick + drift
+  // into second position buffers (EAM passes read gather records and update
+  // in place), as in the single-system scheduler.
+  const bool flips = !eam_ && cfg_.use_graphs != 0;
+  if (flips) {
+    pos4_alt_.reserve(n);
+    if (mixed_) q_alt_.reserve(n);
+  }
   for (int attempt = 0;; ++attempt) {
+    in_alt_ = false;
     TDMD_CU(cudaEventRecord(win_ev_[0], s));
     std::vector<BatchStep> plan;
     int since = since_rebuild_;
@@ -869,14 +902,15 @@ void Batch::run_until(int target) {
       b.rebuild = since >= cfg_.rebuild_every;
       if (b.rebuild) since = 0;
       ++since;
-      // EAM (both precisions): every force pass but the window's last also
-      // kicks and drifts for the next step (energies are logged after the
-      // window)
-      b.fuse_next = eam_ && st + 1 < target;
+      // every force pass but the window's last also kicks and drifts for the
+      // next step (energies are logged after the window)
+      b.fuse_next = (eam_ || flips) && st + 1 < target;
       b.kd_fused = !plan.empty() && plan.back().fuse_next;
       b.log_e = log_now && st + 1 == target;
       plan.push_back(b);
     }
+    // An odd number of buffer changes: the window's first drift makes it even.
+    if (flips && plan.size() % 2 == 0) plan.front().to_alt = true;
     size_t a = 0;
     while (a < plan.size()) {
       size_t b = a + 1;

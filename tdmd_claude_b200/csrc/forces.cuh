@@ -562,6 +562,53 @@ __device__ __forceinline__ void add_virial(double (&w)[6], T fpair, T dx, T dy, 
   w[5] += hf * ddy * ddz;
 }
 
+// The next step's fused kick + drift, applied by a force pass to each atom
+// right after its force: v += dt F/(m mvv2e), x += dt v with the
+// single-image wrap, fixed-point record refreshed (fused_kick_drift_kernel,
+// device_velocity_verlet.cu:88-130, full kick).  The EAM force passes read
+// gather records, never the positions they update; Morse reads the positions
+// themselves, so it writes the new ones to a second buffer (ALT).
+struct KickDrift {
+  double4* pos4;
+  int4* q;
+  double* v;
+  const int* types;
+  const double* inv_mm;  // 1 / (m mvv2e) per type
+  double dt;
+  long long* step;       // device step counter, +1 per kick-drift (nullable)
+  DevBox b;
+  // Batched replicas: atom i's box is reps[rep[i]].box instead of b.
+  const int* rep;
+  const RepDesc* reps;
+  // ALT: where the new positions and fixed-point records go.
+  double4* pos4_alt = nullptr;
+  int4* q_alt = nullptr;
+};
+
+// FT: the force type (float: mixed, also refreshes the fixed-point record;
+// double: FP64, which keeps no fixed-point copy).
+template <bool ALT, class FT>
+__device__ __forceinline__ void kick_drift_atom(const KickDrift& k, int i, FT fx, FT fy, FT fz) {
+  const DevBox& b = k.reps ? k.reps[__ldg(k.rep + i)].box : k.b;
+  const int t = __ldg(k.types + i);
+  const double factor = k.dt * __ldg(k.inv_mm + t);
+  double vx = k.v[3ll * i], vy = k.v[3ll * i + 1], vz = k.v[3ll * i + 2];
+  vx += factor * static_cast<double>(fx);
+  vy += factor * static_cast<double>(fy);
+  vz += factor * static_cast<double>(fz);
+  double4 p = k.pos4[i];
+  p.x = wrap_single(p.x + k.dt * vx, b.lo[0], b.L[0], b.periodic[0]);
+  p.y = wrap_single(p.y + k.dt * vy, b.lo[1], b.L[1], b.periodic[1]);
+  p.z = wrap_single(p.z + k.dt * vz, b.lo[2], b.L[2], b.periodic[2]);
+  k.v[3ll * i] = vx;
+  k.v[3ll * i + 1] = vy;
+  k.v[3ll * i + 2] = vz;
+  (ALT ? k.pos4_alt : k.pos4)[i] = p;
+  if constexpr (sizeof(FT) == sizeof(float))
+    (ALT ? k.q_alt : k.q)[i] = make_int4(encode_q(p.x, b.qlo[0], b.qinv[0]), encode_q(p.y, b.qlo[1], b.qinv[1]),
+                       encode_q(p.z, b.qlo[2], b.qinv[2]), t);
+}
+
 // --------------------------------------------------------------------------
 // Morse, MorsePair::compute (src/potentials/morse.hpp:37-55) on the full
 // list: F_i = sum_j fpair(r_ij) (r_i - r_j), energy 1/2 U per listed pair.
@@ -574,11 +621,16 @@ struct MorseP {
 
 // EV: 0 forces only; 1 also energy + virial into per-block partials and,
 // where pe_atom is given, per-atom energies; 2 forces + per-atom energies.
-template <class Geo, int LPA, int U, int EV, bool VEC, class F, class Out = ForceOut<F>>
+// KD: then the next step's kick + drift of the same atom, the new positions
+// into the second buffers: one launch and one pass over the forces less per
+// step (256 atoms FP64: 672 -> 612 us per 100 steps; 64 replicas, 142k atoms,
+// mixed: 1 %).
+template <class Geo, int LPA, int U, int EV, bool VEC, class F, class Out = ForceOut<F>,
+          bool KD = false>
 __global__ void __launch_bounds__(256) k_morse(Geo g, NbrView nl, int n,
                                                MorseP<typename Geo::T> mp, Out out,
                                                double* __restrict__ partials,
-                                               double* __restrict__ pe_atom) {
+                                               double* __restrict__ pe_atom, KickDrift kd = {}) {
   dependent_launch_prologue();
   using T = typename Geo::T;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -630,7 +682,13 @@ __global__ void __launch_bounds__(256) k_morse(Geo g, NbrView nl, int n,
     fy.shfl_merge(o);
     fz.shfl_merge(o);
   }
-  if (active && sub == 0) out.store(i, fx.value(), fy.value(), fz.value());
+  if (active && sub == 0) {
+    out.store(i, fx.value(), fy.value(), fz.value());
+    if constexpr (KD)
+      kick_drift_atom<true>(kd, i, static_cast<F>(fx.value()), static_cast<F>(fy.value()),
+                            static_cast<F>(fz.value()));
+  }
+  if (KD && kd.step && blockIdx.x == 0 && threadIdx.x == 0) *kd.step += 1;
   if (EV) {
     // per-atom energy (nullable): the lanes' sums merged pairwise
     if (pe_atom) {
@@ -906,49 +964,6 @@ __global__ void __launch_bounds__(256) k_eam_density(Geo g, NbrView nl, int n,
   }
 }
 
-// The next step's fused kick + drift, applied by a force pass to each atom
-// right after its force: v += dt F/(m mvv2e), x += dt v with the
-// single-image wrap, fixed-point record refreshed (fused_kick_drift_kernel,
-// device_velocity_verlet.cu:88-130, full kick).  Only for a force pass that
-// reads gather records, never the positions it updates.
-struct KickDrift {
-  double4* pos4;
-  int4* q;
-  double* v;
-  const int* types;
-  const double* inv_mm;  // 1 / (m mvv2e) per type
-  double dt;
-  long long* step;       // device step counter, +1 per kick-drift (nullable)
-  DevBox b;
-  // Batched replicas: atom i's box is reps[rep[i]].box instead of b.
-  const int* rep;
-  const RepDesc* reps;
-};
-
-// FT: the force type (float: mixed, also refreshes the fixed-point record;
-// double: FP64, which keeps no fixed-point copy).
-template <class FT>
-__device__ __forceinline__ void kick_drift_atom(const KickDrift& k, int i, FT fx, FT fy, FT fz) {
-  const DevBox& b = k.reps ? k.reps[__ldg(k.rep + i)].box : k.b;
-  const int t = __ldg(k.types + i);
-  const double factor = k.dt * __ldg(k.inv_mm + t);
-  double vx = k.v[3ll * i], vy = k.v[3ll * i + 1], vz = k.v[3ll * i + 2];
-  vx += factor * static_cast<double>(fx);
-  vy += factor * static_cast<double>(fy);
-  vz += factor * static_cast<double>(fz);
-  double4 p = k.pos4[i];
-  p.x = wrap_single(p.x + k.dt * vx, b.lo[0], b.L[0], b.periodic[0]);
-  p.y = wrap_single(p.y + k.dt * vy, b.lo[1], b.L[1], b.periodic[1]);
-  p.z = wrap_single(p.z + k.dt * vz, b.lo[2], b.L[2], b.periodic[2]);
-  k.v[3ll * i] = vx;
-  k.v[3ll * i + 1] = vy;
-  k.v[3ll * i + 2] = vz;
-  k.pos4[i] = p;
-  if constexpr (sizeof(FT) == sizeof(float))
-    k.q[i] = make_int4(encode_q(p.x, b.qlo[0], b.qinv[0]), encode_q(p.y, b.qlo[1], b.qinv[1]),
-                       encode_q(p.z, b.qlo[2], b.qinv[2]), t);
-}
-
 // Pass 3: f_ij = -(phi' + fp_i rho'_tj + fp_j rho'_ti)/r * (r_i - r_j).
 // FPG: F'(rho_j) comes with the neighbor's gather record (pair w bits)
 // instead of the fp array.  KD (FPG, float forces): then the next step's
@@ -1051,7 +1066,7 @@ __global__ void __launch_bounds__(256) k_eam_force(Geo g, NbrView nl, int n,
     out.store(i, fx.value(), fy.value(), fz.value());
     if constexpr (KD) {
       static_assert(FPG, "fused kick-drift: a force pass that reads gather records");
-      kick_drift_atom(kd, i, static_cast<F>(fx.value()), static_cast<F>(fy.value()),
+      kick_drift_atom<false>(kd, i, static_cast<F>(fx.value()), static_cast<F>(fy.value()),
                       static_cast<F>(fz.value()));
     }
   }

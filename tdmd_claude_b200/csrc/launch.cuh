@@ -67,22 +67,32 @@ struct Tune {
   TDMD_NU_DISPATCH((tn).nu, TDMD_LPA_DISPATCH((tn).lpa, __VA_ARGS__))
 
 // Morse forces; with ev, per-block partials (force_blocks records; nullable)
-// and per-atom energies (pe_atom, nullable).
-template <class Geo, class F>
+// and per-atom energies (pe_atom, nullable).  kd (nullable, not with ev; FUSE):
+// also the next step's kick + drift into kd's second buffers.
+template <bool FUSE = false, class Geo, class F>
 void launch_morse(const Geo& g, const NbrView& nl, int n, const MorseP<typename Geo::T>& mp,
                   F* forces, bool ev, double* partials, Tune tn, cudaStream_t s,
-                  double* pe_atom = nullptr) {
+                  double* pe_atom = nullptr, const KickDrift* kd = nullptr) {
   const int nblk = force_blocks(n, tn.lpa);
   TDMD_VEC_DISPATCH(vec_rows(nl), TDMD_TUNE_DISPATCH(tn, {
     if (ev && !partials && pe_atom)  // per-atom energies only
       launch(k_morse<Geo, L, U, 2, V, F>, nblk, kForceThreads, 0, s, g, nl, n, mp,
-             ForceOut<F>{forces}, nullptr, pe_atom);
+             ForceOut<F>{forces}, nullptr, pe_atom, KickDrift{});
     else if (ev)
       launch(k_morse<Geo, L, U, 1, V, F>, nblk, kForceThreads, 0, s, g, nl, n, mp,
-             ForceOut<F>{forces}, partials, pe_atom);
-    else
+             ForceOut<F>{forces}, partials, pe_atom, KickDrift{});
+    else if constexpr (FUSE) {
+      if (kd)
+        launch(k_morse<Geo, L, U, 0, V, F, ForceOut<F>, true>, nblk, kForceThreads, 0, s, g, nl,
+               n, mp, ForceOut<F>{forces}, nullptr, nullptr, *kd);
+      else
+        launch(k_morse<Geo, L, U, 0, V, F>, nblk, kForceThreads, 0, s, g, nl, n, mp,
+               ForceOut<F>{forces}, nullptr, nullptr, KickDrift{});
+    } else {
+      TDMD_REQUIRE(kd == nullptr, "fused kick-drift was not asked for");
       launch(k_morse<Geo, L, U, 0, V, F>, nblk, kForceThreads, 0, s, g, nl, n, mp,
-             ForceOut<F>{forces}, nullptr, nullptr);
+             ForceOut<F>{forces}, nullptr, nullptr, KickDrift{});
+    }
   }));
   TDMD_LAUNCH_CHECK();
 }
@@ -101,10 +111,10 @@ void launch_morse_zone(const Geo& g, int first, const NbrView& nl, int n,
   TDMD_LPA_DISPATCH(lpa, {
     if (ev)
       launch(k_morse<GeoShift<Geo>, L, kU, 1, false, F, ForceAdd<F>>, nblk, kForceThreads, 0, s,
-             gs, nl, n, mp, out, partials, nullptr);
+             gs, nl, n, mp, out, partials, nullptr, KickDrift{});
     else
       launch(k_morse<GeoShift<Geo>, L, kU, 0, false, F, ForceAdd<F>>, nblk, kForceThreads, 0, s,
-             gs, nl, n, mp, out, nullptr, nullptr);
+             gs, nl, n, mp, out, nullptr, nullptr, KickDrift{});
   });
   TDMD_LAUNCH_CHECK();
 }

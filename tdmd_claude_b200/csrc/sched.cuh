@@ -46,6 +46,7 @@ struct StepPlan {
   bool ev;         // energy-log step
   bool kd_fused;   // this step's kick + drift ran inside the previous force pass
   bool fuse_next;  // this step's force pass also kicks and drifts for the next step
+  bool to_alt;     // the kick + drift launch writes to the second position buffers
 };
 
 enum ProfCat : int {
@@ -129,12 +130,22 @@ class Scheduler {
   // parts: which EAM passes (density, pair force); Morse has one pass.
   static constexpr int kPassDensity = 1, kPassForce = 2, kPassBoth = 3;
   void enqueue_force(bool ev, bool kd = false, int parts = kPassBoth);
-  // The EAM force passes of both precisions read gather records, never the
-  // positions, so they can carry the next step's kick + drift (NVE only).
-  bool can_fuse_kick() const { return kind_ == TDMD_POT_EAM && !thermo_; }
+  // NVE force passes can carry the next step's kick + drift: the EAM passes of
+  // both precisions read gather records, never the positions; Morse writes
+  // the new positions to the second buffers (graph windows only: launched one
+  // by one, its steps stay the two phases that the launch counts report).
+  bool can_fuse_kick() const {
+    return !thermo_ && (kind_ == TDMD_POT_EAM || cfg_.use_graphs != 0);
+  }
+  // The buffers that hold the positions now.  Fused Morse passes alternate;
+  // a window with an odd number of them starts by drifting into the second
+  // buffers, so that every window ends in the first.
+  bool fused_flips() const { return kind_ == TDMD_POT_MORSE; }
+  double4* pos4() const { return in_alt_ ? pos4_alt_.data() : pos4_.data(); }
+  int4* q() const { return in_alt_ ? q_alt_.data() : q_.data(); }
   template <class F>
-  void enqueue_kick_drift_t(F* f, bool full, bool scale);
-  void enqueue_kick_drift(bool full, bool scale);
+  void enqueue_kick_drift_t(F* f, bool full, bool scale, bool to_alt);
+  void enqueue_kick_drift(bool full, bool scale, bool to_alt = false);
   template <class F>
   void enqueue_half_kick_t(F* f, bool ke);
   void enqueue_half_kick(bool ke);
@@ -193,12 +204,14 @@ class Scheduler {
   DevArray<double> f64_;
   DevArray<float> f32_;
   DevArray<int> types_, ids_;
-  // second buffers of the per-atom state: upload gathers into them and swaps
+  // second buffers of the per-atom state: upload gathers into them and swaps;
+  // inside a window, fused Morse passes alternate between the two
   DevArray<double4> pos4_alt_;
   DevArray<int4> q_alt_;
   DevArray<double> vel_alt_, f64_alt_;
   DevArray<float> f32_alt_;
   DevArray<int> types_alt_, ids_alt_;
+  bool in_alt_ = false;  // inside a window: the positions are in the second buffers
   bool cells_from_upload_ = false;  // cl_ holds the cells of the reordered upload
   DevArray<double> masses_;
   DevArray<double> inv_mm_;  // 1 / (m mvv2e) per type: the kick factor per unit dt

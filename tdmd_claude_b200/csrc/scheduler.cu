@@ -153,8 +153,9 @@ __global__ void __launch_bounds__(kThreads) k_window_prologue(
 // single-image wrap + fixed-point refresh.  fused_kick_drift_kernel,
 // device_velocity_verlet.cu:88-130.  dt comes from the control block when
 // `ctl_dt` (adaptive dt), else from the argument.
+// pos4_out may be pos4 (each thread reads its atom before it writes it).
 template <class F, bool FULL, bool SCALE>
-__global__ void __launch_bounds__(kThreads) k_kick_drift(double4* __restrict__ pos4,
+__global__ void __launch_bounds__(kThreads) k_kick_drift(const double4* pos4, double4* pos4_out,
                                                          int4* __restrict__ q,
                                                          double* __restrict__ v,
                                                          const F* __restrict__ f,
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(kThreads) k_kick_drift(double4* __restrict__ p
   v[3ll * i] = vx;
   v[3ll * i + 1] = vy;
   v[3ll * i + 2] = vz;
-  pos4[i] = p;
+  pos4_out[i] = p;
   if (q)
     q[i] = make_int4(encode_q(p.x, b.qlo[0], b.qinv[0]), encode_q(p.y, b.qlo[1], b.qinv[1]),
                      encode_q(p.z, b.qlo[2], b.qinv[2]), t);
@@ -528,6 +529,7 @@ void Scheduler::upload(const double* x, const double* v, const void* f, const in
   }
   n_types_ = n_types;
   uploaded_ = false;
+  in_alt_ = false;
   cells_from_upload_ = false;
   // Masses, kick factors and the control block through the pinned block
   // (the previous upload's copies from it finished at its synchronisation).
@@ -744,7 +746,7 @@ int Scheduler::build_cells() {
     TDMD_LAUNCH_CHECK();
     return 1;
   }
-  build_cell_list(cl_, pos4_.data(), PosLayout::D4, n_, box_, stream_, order_.data());
+  build_cell_list(cl_, pos4(), PosLayout::D4, n_, box_, stream_, order_.data());
   return cell_list_kernels();
 }
 
@@ -780,7 +782,7 @@ void Scheduler::enqueue_rebuild() {
   prof_begin(kProfRebuild);
   const int cell_kernels = build_cells();
   const double rl = cutoff_ + cfg_.r_skin;
-  build_neighbor_rows(cl_, pos4_.data(), PosLayout::D4, n_, box_, rl * rl, nbr_.data(), nullptr,
+  build_neighbor_rows(cl_, pos4(), PosLayout::D4, n_, box_, rl * rl, nbr_.data(), nullptr,
                       cap_, cnt_.data(), ctl_status(), s, max_cell_);
   prof_end(kProfRebuild);
   launches_ += cell_kernels + 1;  // cell list + row build
@@ -789,7 +791,7 @@ void Scheduler::enqueue_rebuild() {
 
 // ----- forces ---------------------------------------------------------------
 void Scheduler::enqueue_force(bool ev, bool kd, int parts) {
-  TDMD_REQUIRE(!kd || can_fuse_kick(), "fused kick-drift needs the EAM NVE path");
+  TDMD_REQUIRE(!kd || can_fuse_kick(), "fused kick-drift needs an NVE window");
   cudaStream_t s = stream_;
   const NbrView nl{nbr_.data(), nullptr, cnt_.data(), cap_};
   const int nblk = force_blocks(n_, lpa_);       // pair-force pass records
@@ -798,13 +800,29 @@ void Scheduler::enqueue_force(bool ev, bool kd, int parts) {
   double* part = ev ? ev_part_.data() : nullptr;
   if (kind_ == TDMD_POT_MORSE) {
     prof_begin(kProfForce);
+    const KickDrift kdr{pos4(),
+                        nullptr,
+                        vel_.data(),
+                        types_.data(),
+                        inv_mm_.data(),
+                        cfg_.dt,
+                        reinterpret_cast<long long*>(reinterpret_cast<char*>(ctl_.data()) +
+                                                     offsetof(SchedCtl, step)),
+                        box_,
+                        nullptr,
+                        nullptr,
+                        in_alt_ ? pos4_.data() : pos4_alt_.data(),
+                        in_alt_ ? q_.data() : q_alt_.data()};
     if (mixed_) {
-      const GeoQ g = make_geoq(q_.data(), box_);
-      launch_morse(g, nl, n_, m32_, f32_.data(), ev, part, tf, s);
+      const GeoQ g = make_geoq(q(), box_);
+      launch_morse<true>(g, nl, n_, m32_, f32_.data(), ev, part, tf, s, nullptr,
+                         kd ? &kdr : nullptr);
     } else {
-      const GeoD4 g{pos4_.data(), img3(box_)};
-      launch_morse(g, nl, n_, m64_, f64_.data(), ev, part, tf, s);
+      const GeoD4 g{pos4(), img3(box_)};
+      launch_morse<true>(g, nl, n_, m64_, f64_.data(), ev, part, tf, s, nullptr,
+                         kd ? &kdr : nullptr);
     }
+    if (kd) in_alt_ = !in_alt_;
     prof_end(kProfForce);
     launches_ += 1;
   } else {
@@ -872,30 +890,33 @@ void Scheduler::enqueue_force(bool ev, bool kd, int parts) {
 
 // ----- integration ----------------------------------------------------------
 template <class F>
-void Scheduler::enqueue_kick_drift_t(F* f, bool full, bool scale) {
+void Scheduler::enqueue_kick_drift_t(F* f, bool full, bool scale, bool to_alt) {
   cudaStream_t s = stream_;
   const int nb = ceil_div(n_, kThreads);
-  int4* q = mixed_ ? q_.data() : nullptr;
+  double4* const from = pos4();
+  if (to_alt) in_alt_ = !in_alt_;
+  double4* const to = pos4();
+  int4* q = mixed_ ? this->q() : nullptr;
   const int ctl_dt = thermo_ ? 1 : 0;
   if (scale)
-    launch(k_kick_drift<F, false, true>, nb, kThreads, 0, s, pos4_.data(), q, vel_.data(), f,
+    launch(k_kick_drift<F, false, true>, nb, kThreads, 0, s, from, to, q, vel_.data(), f,
            types_.data(), inv_mm_.data(), n_, cfg_.dt, ctl_.data(), ctl_dt, box_);
   else if (full)
-    launch(k_kick_drift<F, true, false>, nb, kThreads, 0, s, pos4_.data(), q, vel_.data(), f,
+    launch(k_kick_drift<F, true, false>, nb, kThreads, 0, s, from, to, q, vel_.data(), f,
            types_.data(), inv_mm_.data(), n_, cfg_.dt, ctl_.data(), ctl_dt, box_);
   else
-    launch(k_kick_drift<F, false, false>, nb, kThreads, 0, s, pos4_.data(), q, vel_.data(), f,
+    launch(k_kick_drift<F, false, false>, nb, kThreads, 0, s, from, to, q, vel_.data(), f,
            types_.data(), inv_mm_.data(), n_, cfg_.dt, ctl_.data(), ctl_dt, box_);
   TDMD_LAUNCH_CHECK();
   launches_ += 1;
 }
 
-void Scheduler::enqueue_kick_drift(bool full, bool scale) {
+void Scheduler::enqueue_kick_drift(bool full, bool scale, bool to_alt) {
   prof_begin(kProfKickDrift);
   if (mixed_)
-    enqueue_kick_drift_t(f32_.data(), full, scale);
+    enqueue_kick_drift_t(f32_.data(), full, scale, to_alt);
   else
-    enqueue_kick_drift_t(f64_.data(), full, scale);
+    enqueue_kick_drift_t(f64_.data(), full, scale, to_alt);
   prof_end(kProfKickDrift);
 }
 
@@ -983,7 +1004,7 @@ void Scheduler::enqueue_apply_scale() {
 // One step as planned (see plan_steps): the kernels of the step.
 void Scheduler::enqueue_step(const StepPlan& st) {
   if (!thermo_) {
-    if (!st.kd_fused) enqueue_kick_drift(/*full=*/!st.first, /*scale=*/false);
+    if (!st.kd_fused) enqueue_kick_drift(/*full=*/!st.first, /*scale=*/false, st.to_alt);
     if (st.rebuild) enqueue_rebuild();
     enqueue_force(st.ev, st.fuse_next);
     if (st.ev) enqueue_log_nve();
@@ -1022,10 +1043,14 @@ void Scheduler::run_segment(const std::vector<StepPlan>& seg, bool finalize, int
   key.reserve(seg.size() + 2);
   for (const auto& st : seg)
     key.push_back((st.first ? 1 : 0) | (st.rebuild ? 2 : 0) | (st.ev ? 4 : 0) | (st.last ? 8 : 0) |
-                  (st.kd_fused ? 16 : 0) | (st.fuse_next ? 32 : 0));
+                  (st.kd_fused ? 16 : 0) | (st.fuse_next ? 32 : 0) | (st.to_alt ? 64 : 0));
   key.push_back(finalize ? 1 : 0);
   key.push_back(prologue);
   key.push_back(profiling_ ? 1 : 0);
+  key.push_back(in_alt_ ? 1 : 0);
+  bool end_in_alt = in_alt_;  // where the segment leaves the positions
+  for (const auto& st : seg)
+    end_in_alt = end_in_alt != (st.to_alt != (st.fuse_next && fused_flips()));
   const long long l0 = launches_;
   if (!cfg_.use_graphs) {
     enqueue_prologue(prologue);
@@ -1052,12 +1077,14 @@ void Scheduler::run_segment(const std::vector<StepPlan>& seg, bool finalize, int
       prof_sink_ = &ge.prof;
       suppress_programmatic_launch(true);
     }
+    const bool start_in_alt = in_alt_;
     TDMD_CU(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     try {
       enqueue_prologue(prologue);
       for (const auto& st : seg) enqueue_step(st);
       if (finalize) enqueue_finalize();
     } catch (...) {
+      in_alt_ = start_in_alt;
       prof_sink_ = nullptr;
       suppress_programmatic_launch(false);
       cudaStreamEndCapture(stream_, &g);
@@ -1080,6 +1107,7 @@ void Scheduler::run_segment(const std::vector<StepPlan>& seg, bool finalize, int
     graph_lru_.push_front(key);
   }
   TDMD_CU(cudaGraphLaunch(it->second.exec, stream_));
+  in_alt_ = end_in_alt;
   launches_ += it->second.kernels;
   ++graph_launches_;
   for (const ProfEvents& pe : it->second.prof) prof_graph_pending_.push_back(pe);
@@ -1099,11 +1127,17 @@ std::vector<StepPlan> Scheduler::plan_steps(int target, int* since_out) const {
     if (st.rebuild) since = 0;
     ++since;
     st.ev = cfg_.energy_every > 0 && ((s + 1) % cfg_.energy_every == 0);
-    // Mixed EAM NVE: a force pass that logs no energy and is followed by
-    // another step of the window also kicks and drifts for that step.
+    // NVE: a force pass that logs no energy and is followed by another step
+    // of the window also kicks and drifts for that step.
     st.fuse_next = can_fuse_kick() && !st.ev && !st.last;
     st.kd_fused = !plan.empty() && plan.back().fuse_next;
     plan.push_back(st);
+  }
+  // An odd number of buffer changes: the window's first drift makes it even.
+  if (fused_flips()) {
+    long long fused = 0;
+    for (const auto& st : plan) fused += st.fuse_next ? 1 : 0;
+    if (fused % 2) plan.front().to_alt = true;
   }
   *since_out = since;
   return plan;
@@ -1207,6 +1241,7 @@ void Scheduler::run_until(int target) {
   const int step0 = step_, since0 = since_rebuild_;
   reserve_snapshot();
   for (int attempt = 0;; ++attempt) {
+    in_alt_ = false;
     TDMD_CU(cudaEventRecord(win_ev_[0], stream_));
     // The snapshot and the flag reset go into the first segment's graph: one
     // submission per window.  A pending first-list overflow flag stays set

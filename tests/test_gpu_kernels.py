@@ -188,3 +188,41 @@ def test_cell_list_one_block(cuda, oracle, n, nc):
     enc, ecc, eco, eca, eac = want
     for g, w in zip(got, (enc, eca, eco, ecc, eac)):
         assert np.array_equal(g, w)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("energy_every", [0, 3])
+@pytest.mark.parametrize("batch", [False, True])
+def test_morse_fused_kick_equals_unfused(cuda, precision, energy_every, batch):
+    """Morse graph windows drift inside the force pass, into a second position
+    buffer; windows launched one by one do not.  Windows of one step, of odd
+    and even lengths, across rebuilds and past one graph segment, with and
+    without energy-log steps: the same bits, and energies of the state that
+    each window leaves."""
+    from tdmd_claude_b200 import (Box, FastPipelineScheduler, MorseParams, ReplicaBatch,
+                                  make_config)
+    from tdmd_claude_b200 import workloads as W
+    s = W.fcc_system(4, 3.615, 600.0, 3)
+    out = []
+    for graphs in (True, False):
+        cfg = make_config(r_skin=0.3, rebuild_every=70, precision=precision, lanes_per_atom=8,
+                          use_graphs=graphs, energy_every=energy_every, energy_log_capacity=256)
+        p = MorseParams.make(*W.MORSE_CU)
+        if batch:
+            m = ReplicaBatch([Box.make(s.lo, s.hi)] * 2, [s.n, s.n], p, cfg)
+            m.upload(np.concatenate([s.positions, s.positions]),
+                     np.concatenate([s.velocities, 0.5 * s.velocities]),
+                     np.concatenate([s.types] * 2), s.masses)
+        else:
+            m = FastPipelineScheduler(Box.make(s.lo, s.hi), s.n, p, cfg)
+            m.upload(s.positions, s.velocities, None, s.types, s.ids, s.masses)
+        for t in (1, 3, 6, 16, 27, 160, 161):
+            m.run_until(t)
+            st = m.download()
+            out.append([*(st if batch else (st.positions, st.velocities, st.forces)),
+                        *m.energies()])
+        m.close()
+    half = len(out) // 2
+    for a, b in zip(out[:half], out[half:]):
+        for x, y in zip(a, b):
+            assert np.array_equal(x, y)
