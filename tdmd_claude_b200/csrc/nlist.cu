@@ -377,7 +377,10 @@ __device__ __forceinline__ void build_cell_rows(
   const unsigned lt_mask = (1u << lane) - 1u;
   const float Lx = static_cast<float>(b.L[0]), Ly = static_cast<float>(b.L[1]),
               Lz = static_cast<float>(b.L[2]);
-  const float hx = 0.5f * Lx, hy = 0.5f * Ly, hz = 0.5f * Lz;
+  // half extents of the FP32 re-wrap; +infinity on a free axis
+  const float hx = b.periodic[0] ? 0.5f * Lx : INFINITY;
+  const float hy = b.periodic[1] ? 0.5f * Ly : INFINITY;
+  const float hz = b.periodic[2] ? 0.5f * Lz : INFINITY;
   int wmax = 0;  // lane 0: this warp's longest row
   // The row of one center atom (record ci, candidate index self_k) over
   // candidates cand(0 .. nloop): padded sources carry sentinels up to whole
@@ -390,17 +393,54 @@ __device__ __forceinline__ void build_cell_rows(
                                    : static_cast<long long>(i) * cap;
     const int limit = row_off ? INT_MAX : cap;
     int cnt = 0;
+    auto dist2 = [&](const float4& cj) {
+      float dx = __fsub_rn(cj.x, ci.x), dy = __fsub_rn(cj.y, ci.y), dz = __fsub_rn(cj.z, ci.z);
+      if (WRAP) {
+        dx = fabsf(dx) > hx ? dx - copysignf(Lx, dx) : dx;
+        dy = fabsf(dy) > hy ? dy - copysignf(Ly, dy) : dy;
+        dz = fabsf(dz) > hz ? dz - copysignf(Lz, dz) : dz;
+      }
+      return r2_rn(dx, dy, dz);
+    };
+    // Fast row (replica kernel): the filter alone, noting whether any candidate
+    // falls into the band (about one row in a hundred); such a row is swept
+    // again with the exact test below.  The band is voted on once a row instead
+    // of once a sweep: 64 Morse replicas, 142k atoms, 247 -> 180 us a build.  (A
+    // row that is swept again only gains entries, so it never writes past its
+    // end.)  The single-system kernel, whose sweeps are shorter and wait on its
+    // staging, gained nothing (118k atoms: 165 us either way) and lost 2 % on
+    // 2 767 atoms.
+    if constexpr (kPadded && SLAB) {
+      int* const out = WRITE ? nbr + base : nullptr;
+      bool band = false;
+#pragma unroll 2
+      for (int k0 = 0; k0 < nloop; k0 += 32) {
+        const float4 cj = cand(k0 + lane);
+        const int j = __float_as_int(cj.w);
+        const float r2f = dist2(cj);
+        const bool in = r2f < lo_f && j != i;
+        band = band || (!(r2f < lo_f) && !(r2f > hi_f));
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (WRITE) {
+          const int p = cnt + __popc(m & lt_mask);
+          if (in && p < limit) out[p] = j;
+        }
+        cnt += __popc(m);
+      }
+      if (!__any_sync(0xffffffffu, band)) {
+        if (lane == 0) {
+          counts[i] = cnt;
+          wmax = cnt > wmax ? cnt : wmax;
+        }
+        return;
+      }
+      cnt = 0;
+    }
     for (int k0 = 0; k0 < nloop; k0 += 32) {
       const int k = k0 + lane;
       const float4 cj = cand(kPadded ? k : (k < nloop ? k : self_k));
       const int j = __float_as_int(cj.w);
-      float dx = __fsub_rn(cj.x, ci.x), dy = __fsub_rn(cj.y, ci.y), dz = __fsub_rn(cj.z, ci.z);
-      if (WRAP) {
-        dx = min_image1(dx, Lx, hx, b.periodic[0]);
-        dy = min_image1(dy, Ly, hy, b.periodic[1]);
-        dz = min_image1(dz, Lz, hz, b.periodic[2]);
-      }
-      const float r2f = r2_rn(dx, dy, dz);
+      const float r2f = dist2(cj);
       const bool other = j != i;
       unsigned m = __ballot_sync(0xffffffffu, other && r2f < lo_f);
       // Candidates inside the filter's band go to the exact FP64 test:
