@@ -107,10 +107,9 @@ __global__ void __launch_bounds__(kThreads) k_eam_atom_pe(Geo g, NbrView nl, int
         typename Geo::Pair pr;
         g.pair(o, jj[u], pr);
         if (pr.r2 < e.rc_sq) {
-          T r, rinv, sx;
-          double rd;
-          g.radius(o, pr, r, rinv, rd);
-          const int idx = spline_at(r, rd, e.dr, e.inv_dr, e.nr, e.dr_d, sx);
+          T r, rinv, corr, sx;
+          g.radius2(o, pr, r, rinv, corr);
+          const int idx = spline_at(r, corr, e, sx);
           const int tj = MULTI ? __ldg(types + jj[u]) - 1 : 0;
           const auto cphi = ldv4<T>(e.rtab + static_cast<long long>(idx) * e.S +
                                     (MULTI ? phi_slot(ti, tj, e.ntypes) : 1));

@@ -234,6 +234,15 @@ struct PairQ {
 // |r| and 1/|r| in FP32 and the FP64-refined radius from a PairQ: with
 // r = sqrt(r2) in FP32, r2d - r*r = res + (r2 - r*r), the second term exact
 // by FMA; one Newton step rd = r + (r2d - r*r) / (2r).
+// 1/sqrt of a fixed-point pair's r^2: zero or at least (L/2^32)^2, so the
+// reciprocal root needs none of rsqrtf's rescaling of subnormals (two
+// predicated multiplications and a compare a pair; same bits).
+__device__ __forceinline__ float rsqrt_q(float r2) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(r2));
+  return y;
+}
+
 // FP64 residual (exact r^2 of the fixed-point deltas) - r2.  When the
 // three axes share one step (iso), the squares are summed exactly in 64-bit
 // integers (|d| <= 2^31: each square <= 2^62, the sum < 2^64) and scaled
@@ -251,10 +260,24 @@ __device__ __forceinline__ float q_residual(int ix, int iy, int iz, int iso, dou
 }
 
 __device__ __forceinline__ void radius_q(float r2, float res, float& r, float& rinv, double& rd) {
-  rinv = rsqrtf(r2);
+  rinv = rsqrt_q(r2);
   r = r2 * rinv;
   const float corr = (res + fmaf(-r, r, r2)) * 0.5f * rinv;
   rd = static_cast<double>(r) + static_cast<double>(corr);
+}
+
+// The same refined radius as a pair of floats r + corr.
+__device__ __forceinline__ void radius_q2(float r2, float res, float& r, float& rinv,
+                                          float& corr) {
+  rinv = rsqrt_q(r2);
+  r = r2 * rinv;
+  corr = (res + fmaf(-r, r, r2)) * 0.5f * rinv;
+}
+__device__ __forceinline__ void radius_f2(float r2, double r2d, float& r, float& rinv,
+                                          float& corr) {
+  rinv = rsqrtf(r2);
+  r = r2 * rinv;
+  corr = static_cast<float>(fma(-static_cast<double>(r), r, r2d)) * 0.5f * rinv;
 }
 
 __device__ __forceinline__ void radius_f(float r2, double r2d, float& r, float& rinv, double& rd) {
@@ -296,6 +319,11 @@ struct GeoD4 {  // FP64, scheduler layout double4 {x,y,z,type}
     radius_d(pr.r2, r, rinv);
     rd = r;
   }
+  __device__ __forceinline__ void radius2(const Own&, const Pair& pr, T& r, T& rinv,
+                                          T& corr) const {
+    radius_d(pr.r2, r, rinv);
+    corr = 0.0;
+  }
   __device__ __forceinline__ T radius_fast(const Pair& pr) const {
     T r, rinv;
     radius_d(pr.r2, r, rinv);
@@ -336,6 +364,11 @@ struct GeoD4F {
     radius_d(pr.r2, r, rinv);
     rd = r;
   }
+  __device__ __forceinline__ void radius2(const Own&, const Pair& pr, T& r, T& rinv,
+                                          T& corr) const {
+    radius_d(pr.r2, r, rinv);
+    corr = 0.0;
+  }
   __device__ __forceinline__ T radius_fast(const Pair& pr) const {
     T r, rinv;
     radius_d(pr.r2, r, rinv);
@@ -371,6 +404,11 @@ struct GeoAoS64 {  // FP64, reference Vec3D AoS
                                          double& rd) const {
     radius_d(pr.r2, r, rinv);
     rd = r;
+  }
+  __device__ __forceinline__ void radius2(const Own&, const Pair& pr, T& r, T& rinv,
+                                          T& corr) const {
+    radius_d(pr.r2, r, rinv);
+    corr = 0.0;
   }
   __device__ __forceinline__ T radius_fast(const Pair& pr) const {
     T r, rinv;
@@ -410,6 +448,10 @@ struct GeoAoS32 {
                                          double& rd) const {
     radius_f(pr.r2, pr.r2d, r, rinv, rd);
   }
+  __device__ __forceinline__ void radius2(const Own&, const Pair& pr, T& r, T& rinv,
+                                          T& corr) const {
+    radius_f2(pr.r2, pr.r2d, r, rinv, corr);
+  }
   __device__ __forceinline__ T radius_fast(const Pair& pr) const { return pr.r2 * rsqrtf(pr.r2); }
 };
 
@@ -443,7 +485,11 @@ struct GeoQ {
                                          double& rd) const {
     radius_q(pr.r2, pr.res, r, rinv, rd);
   }
-  __device__ __forceinline__ T radius_fast(const Pair& pr) const { return pr.r2 * rsqrtf(pr.r2); }
+  __device__ __forceinline__ void radius2(const Own&, const Pair& pr, T& r, T& rinv,
+                                          T& corr) const {
+    radius_q2(pr.r2, pr.res, r, rinv, corr);
+  }
+  __device__ __forceinline__ T radius_fast(const Pair& pr) const { return pr.r2 * rsqrt_q(pr.r2); }
   // F'(rho_j) of a gather record: the 4th word's float bits, type bits cleared
   __device__ __forceinline__ float gather_fp(const Pair& pr, int tmask) const {
     return __int_as_float(pr.w & ~tmask);
@@ -778,16 +824,36 @@ __device__ __forceinline__ int spline_idx_mul(double r, double dr, double inv_dr
   return idx;
 }
 
-// Interval from r in T, offset from the FP64 radius.
-__device__ __forceinline__ int spline_at(double r, double /*rd*/, double dr, double inv_dr,
-                                         int n, double /*dr_d*/, double& sx) {
-  return spline_idx_mul(r, dr, inv_dr, n, sx);
+// Interval of r in FP32 and the same number as a float, as spline_idx_mul has
+// it in FP64: no conversions, which run at a quarter of the rate of the
+// additions that replace them.  0 <= r / dr < 2^22.
+__device__ __forceinline__ int spline_interval(float r, const EamDev<float>& e, float& fi) {
+  constexpr float kRound = 12582912.f;  // 1.5 * 2^23
+  const float z = __fadd_rn(fmaf(r, e.inv_dr, -0.5f), kRound);
+  int idx = __float_as_int(z) - 0x4B400000;
+  fi = __fsub_rn(z, kRound);
+  if (static_cast<unsigned>(idx) > static_cast<unsigned>(e.nr - 2)) {
+    idx = idx < 0 ? 0 : e.nr - 2;
+    fi = static_cast<float>(idx);
+  }
+  return idx;
 }
-__device__ __forceinline__ int spline_at(float r, double rd, float /*dr*/, float inv_dr, int n,
-                                         double dr_d, float& sx) {
-  int idx = static_cast<int>(r * inv_dr);
-  idx = idx < 0 ? 0 : (idx > n - 2 ? n - 2 : idx);
-  sx = static_cast<float>(fma(-static_cast<double>(idx), dr_d, rd));
+
+// Interval from r, offset from the refined radius r + corr (FP32: the knot
+// spacing as dr + dr_lo, so that the offset rounds at its own size, below
+// 2e-10 A).  Without the FP64 radius, whose four conversions and two FP64
+// operations a pair sat in the chain from distance to spline row, and with the
+// intervals above: mixed EAM 131k 3.84 -> 3.81 ms per 50 steps, 1.05 M atoms
+// 11.81 -> 11.59 ms per 20, ternary 55k NVT 3.06 -> 2.97 ms per 50; 2 767 atoms
+// within the spread of its launch shapes (1.14-1.19 ms).
+__device__ __forceinline__ int spline_at(double r, double /*corr*/, const EamDev<double>& e,
+                                         double& sx) {
+  return spline_idx_mul(r, e.dr, e.inv_dr, e.nr, sx);
+}
+__device__ __forceinline__ int spline_at(float r, float corr, const EamDev<float>& e, float& sx) {
+  float fi;
+  const int idx = spline_interval(r, e, fi);
+  sx = __fadd_rn(fmaf(-fi, e.dr, r), fmaf(-fi, e.dr_lo, corr));
   return idx;
 }
 
@@ -798,9 +864,8 @@ __device__ __forceinline__ int spline_fast(double r, const EamDev<T>& e, double&
 }
 template <class T>
 __device__ __forceinline__ int spline_fast(float r, const EamDev<T>& e, float& sx) {
-  int idx = static_cast<int>(r * e.inv_dr);
-  idx = idx < 0 ? 0 : (idx > e.nr - 2 ? e.nr - 2 : idx);
-  const float fi = static_cast<float>(idx);
+  float fi;
+  const int idx = spline_interval(r, e, fi);
   sx = fmaf(-fi, e.dr_lo, fmaf(-fi, e.dr, r));
   return idx;
 }
@@ -1014,10 +1079,9 @@ __global__ void __launch_bounds__(256) k_eam_force(Geo g, NbrView nl, int n,
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (pr[u].r2 < e.rc_sq) {
-          T r, rinv, sx;
-          double rd;
-          g.radius(o, pr[u], r, rinv, rd);
-          const int idx = spline_at(r, rd, e.dr, e.inv_dr, e.nr, e.dr_d, sx);
+          T r, rinv, corr, sx;
+          g.radius2(o, pr[u], r, rinv, corr);
+          const int idx = spline_at(r, corr, e, sx);
           const int j = jj[u];
           int tj = 0;
           if constexpr (MULTI && FPG && Geo::kRecords)

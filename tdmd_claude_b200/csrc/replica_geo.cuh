@@ -55,7 +55,11 @@ struct GeoQB {
                                          double& rd) const {
     radius_q(pr.r2, pr.res, r, rinv, rd);
   }
-  __device__ __forceinline__ T radius_fast(const Pair& pr) const { return pr.r2 * rsqrtf(pr.r2); }
+  __device__ __forceinline__ void radius2(const Own&, const Pair& pr, T& r, T& rinv,
+                                          T& corr) const {
+    radius_q2(pr.r2, pr.res, r, rinv, corr);
+  }
+  __device__ __forceinline__ T radius_fast(const Pair& pr) const { return pr.r2 * rsqrt_q(pr.r2); }
   // F'(rho_j) of a gather record: the 4th word's float bits, type bits cleared
   __device__ __forceinline__ float gather_fp(const Pair& pr, int tmask) const {
     return __int_as_float(pr.w & ~tmask);
@@ -106,6 +110,11 @@ struct GeoD4B {
     radius_d(pr.r2, r, rinv);
     rd = r;
   }
+  __device__ __forceinline__ void radius2(const Own&, const Pair& pr, T& r, T& rinv,
+                                          T& corr) const {
+    radius_d(pr.r2, r, rinv);
+    corr = 0.0;
+  }
   __device__ __forceinline__ T radius_fast(const Pair& pr) const {
     T r, rinv;
     radius_d(pr.r2, r, rinv);
@@ -139,6 +148,11 @@ struct GeoD4BF {
                                          double& rd) const {
     radius_d(pr.r2, r, rinv);
     rd = r;
+  }
+  __device__ __forceinline__ void radius2(const Own&, const Pair& pr, T& r, T& rinv,
+                                          T& corr) const {
+    radius_d(pr.r2, r, rinv);
+    corr = 0.0;
   }
   __device__ __forceinline__ T radius_fast(const Pair& pr) const {
     T r, rinv;

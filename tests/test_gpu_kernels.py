@@ -226,3 +226,32 @@ def test_morse_fused_kick_equals_unfused(cuda, precision, energy_every, batch):
     for a, b in zip(out[:half], out[half:]):
         for x, y in zip(a, b):
             assert np.array_equal(x, y)
+
+
+# on spline knots (dr = 5/1999), inside an interval, in the last one before the
+# cutoff
+@pytest.mark.parametrize("r", [400 * 5 / 1999, 1000 * 5 / 1999, 2.556, 4.4, 4.9985])
+def test_mixed_pair_interval(cuda, r):
+    """Two atoms r apart in mixed precision: FP32 rounds the distance (6e-8 of
+    it), the offset and about ten products and sums: 1e-6 of the density (and
+    3e-7 A of its slope), 3e-6 of the force's two terms before they cancel."""
+    from tdmd_claude_b200 import Box, DeviceEam, EamAlloy
+    from tdmd_claude_b200 import workloads as W
+    t = W.cu_eam_tables()
+    eam = EamAlloy.from_tables(t.ntypes, t.nrho, t.drho, t.nr, t.dr, t.cutoff, t.F, t.rho, t.rphi)
+    de = DeviceEam()
+    de.upload_tables(eam)
+    pos = np.array([[0.0, 1.0, 2.0], [r, 1.0, 2.0]])
+    f = cuda.zeros((2, 3), dtype=cuda.float32, device="cuda")
+    rho = cuda.zeros(2, dtype=cuda.float64, device="cuda")
+    nbr, off, cnt = (_dev(cuda, np.array(x, np.int32)) for x in ([1, 0], [0, 1], [1, 1]))
+    de.compute(_dev(cuda, pos), f, _dev(cuda, np.ones(2, np.int32)), nbr.data_ptr(),
+               off.data_ptr(), cnt.data_ptr(), 2, Box.make((-10.0,) * 3, (22.0,) * 3), d_rho=rho,
+               precision="mixed")
+    want, drho = _spline(eam.coeffs(1, 0), r, t.dr)
+    assert np.abs(rho.cpu().numpy() - want).max() <= 1e-6 * want + 3e-7 * abs(drho)
+    fp = _spline(eam.coeffs(0, 0), want, t.drho)[1]
+    dphi = _spline(eam.coeffs(2, 0), r, t.dr)[1]
+    wf = (dphi + 2 * fp * drho)  # on atom 0, towards atom 1 when positive
+    bound = 3e-6 * (abs(dphi) + abs(2 * fp * drho)) + 1e-7
+    assert np.abs(f.cpu().numpy()[:, 0] - [wf, -wf]).max() <= bound
