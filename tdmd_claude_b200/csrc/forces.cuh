@@ -17,7 +17,8 @@
 //    difference IS the minimum image (scheduler's mixed path, 16-byte
 //    gathers).
 //  * Mixed precision: FP32 distances/splines/forces with rsqrt-based 1/r,
-//    an FP64-refined radius for the spline offset and the Morse exponent,
+//    a refined radius (two floats for the spline offset, FP64 for the Morse
+//    exponent),
 //    compensated FP32 per-atom sums (Kahan per lane, TwoSum across lanes);
 //    energies and virial always accumulate in FP64.
 //  * Energy/virial (template EV): per-block FP64 partials reduced later in a
@@ -148,8 +149,9 @@ __device__ __forceinline__ void nbr_batch(const NbrView& nl, long long row, int 
 // --------------------------------------------------------------------------
 // Geometry policies.  own(i) loads atom i once; pair(own, j, p) fills p with
 // r_i - r_j after the minimum image and r^2 in the policy's arithmetic type
-// T; radius(own, p, r, rinv, rd) gives |r_i - r_j| and its inverse as T and as an
-// FP64 value rd that the spline offset and the Morse exponent use.  In
+// T; radius(own, p, r, rinv, rd) gives |r_i - r_j| and its inverse as T and as
+// an FP64 value rd that the Morse exponent and the fits use, radius2 the same
+// refined radius as r + corr in T for the spline offset.  In
 // FP32, r itself carries an absolute error of ~ulp(r) = 2.4e-7 A at
 // r ~ 2.5 A, which moves the spline argument and, through the large pair
 // forces that cancel in each atom's net force, dominates the mixed-precision
@@ -769,8 +771,7 @@ struct EamDev {
   int ntypes, S, nr, nrho;
   T dr, inv_dr, rc_sq;
   double drho;
-  double dr_d;
-  // FP32 path: dr_d - dr (the knot spacing's rounding), so that the
+  // FP32 path: the FP64 knot spacing less dr (its rounding), so that the
   // spline offset r - idx*dr carries no error proportional to idx (the
   // same sign for every pair of a neighbor shell, which summed into a
   // bias of the embedding energy).
