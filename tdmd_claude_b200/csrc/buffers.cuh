@@ -57,6 +57,37 @@ class DevArray {
   size_t cap_ = 0;
 };
 
+// Scratch of one call: the caller's kept array, except while the stream is
+// captured, when it is a stream-ordered allocation that belongs to the graph --
+// a capture may not allocate the array, and a later call that grows it would
+// free it under the graph.
+template <class T>
+class CallScratch {
+ public:
+  CallScratch(DevArray<T>& keep, size_t keep_n, size_t n, cudaStream_t s) : s_(s) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    TDMD_CU(cudaStreamIsCapturing(s, &cs));
+    if (cs == cudaStreamCaptureStatusNone) {
+      keep.reserve(keep_n);
+      p_ = keep.data();
+    } else {
+      TDMD_CU(cudaMallocAsync(reinterpret_cast<void**>(&p_), n * sizeof(T), s));
+      owned_ = true;
+    }
+  }
+  ~CallScratch() {
+    if (owned_) cudaFreeAsync(p_, s_);
+  }
+  CallScratch(const CallScratch&) = delete;
+  CallScratch& operator=(const CallScratch&) = delete;
+  T* data() const { return p_; }
+
+ private:
+  T* p_ = nullptr;
+  cudaStream_t s_;
+  bool owned_ = false;
+};
+
 // Device-resident cell list (counting sort of atoms into cells), produced by
 // build_cell_list() in nlist.cu.
 struct CellListDev {

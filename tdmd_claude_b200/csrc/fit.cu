@@ -564,31 +564,6 @@ __global__ void __launch_bounds__(256) k_fm_eam_window(const double* __restrict_
 // (7 doubles each): the top 1280, 70 KiB.
 constexpr int kAdjointWindow = 1280;
 
-// The spline rows of one call: the handle's buffer, except while the stream is
-// captured, when they belong to the graph (a buffer that a later call with
-// larger tables would replace must not be in it).
-struct RowScratch {
-  double4* p = nullptr;
-  cudaStream_t s = nullptr;
-  bool owned = false;
-  RowScratch(DevArray<double4>& keep, size_t n, cudaStream_t st) : s(st) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    TDMD_CU(cudaStreamIsCapturing(st, &cs));
-    if (cs == cudaStreamCaptureStatusNone) {
-      keep.reserve(n);
-      p = keep.data();
-    } else {
-      TDMD_CU(cudaMallocAsync(reinterpret_cast<void**>(&p), n * sizeof(double4), st));
-      owned = true;
-    }
-  }
-  ~RowScratch() {
-    if (owned) cudaFreeAsync(p, s);
-  }
-  RowScratch(const RowScratch&) = delete;
-  RowScratch& operator=(const RowScratch&) = delete;
-};
-
 class Fit {
  public:
   Fit(int nsnap, int natoms, const tdmd_box& box, const double* pos, const int* types,
@@ -820,10 +795,11 @@ void Fit::eam(int ntypes, int nrho, double drho, int nr, double dr, const double
   const bool grad = gF || grho || gphi;
   TDMD_REQUIRE(!grad || (gF && grho && gphi), "give all three gradient arrays or none");
   const int npairs = ntypes * (ntypes + 1) / 2;
-  const RowScratch rows(rows_, static_cast<size_t>(ntypes + npairs) * (nr - 1), s);
-  const FitEam e{F, rows.p, gF, grho, gphi, ntypes, nrho - 1, nr - 1, drho, dr, 1.0 / dr};
+  const size_t nrows = static_cast<size_t>(ntypes + npairs) * (nr - 1);
+  const CallScratch<double4> rows(rows_, nrows, nrows, s);
+  const FitEam e{F, rows.data(), gF, grho, gphi, ntypes, nrho - 1, nr - 1, drho, dr, 1.0 / dr};
   launch(k_fm_rows, std::min(2 * sm_count(), ceil_div(4ll * (ntypes + npairs) * (nr - 1), 256)),
-         256, 0, s, rho, phi, ntypes, npairs, nr - 1, rows.p, gF,
+         256, 0, s, rho, phi, ntypes, npairs, nr - 1, rows.data(), gF,
          4ll * (nrho - 1) * ntypes, grho, gphi);
   TDMD_LAUNCH_CHECK();
   const NbrView nl = view();

@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <fstream>
+#include <optional>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -338,7 +339,9 @@ struct tdmd_device_eam {
   DevArray<float> fp32;
   DevArray<double> fp64;
   // energy/virial block partials: kept, because a pool allocation per call
-  // goes back to the driver at every synchronisation (0.4 to 5 ms to map again)
+  // goes back to the driver at every synchronisation (0.4 to 5 ms to map again).
+  // Sized for 32 lanes an atom: fewer atoms take more lanes and can need more
+  // blocks, so that only this size never shrinks with the atom count.
   DevArray<double> part;
   DevArray<double4> rec;  // FP64 {x, y, z, F'} gather records of the force pass
   // the reference's flat layout, for the ID-ordered energy mode
@@ -589,7 +592,12 @@ int32_t tdmd_device_eam_compute(tdmd_device_eam* de, const double* d_positions, 
     const int lpa = default_lpa(natoms);
     const int nblk = force_blocks(natoms, lpa);
     // Density records [0, nblk) and force records [nblk, 2*nblk).
-    de->part.reserve(static_cast<size_t>(2 * nblk) * kEvStride);
+    std::optional<CallScratch<double>> scratch;
+    if (ev)
+      scratch.emplace(de->part, 2 * static_cast<size_t>(force_blocks(natoms, 32)) * kEvStride,
+                      2 * static_cast<size_t>(nblk) * kEvStride, s);
+    double* const part = ev ? scratch->data() : nullptr;
+    double* const part_f = ev ? part + static_cast<long long>(nblk) * kEvStride : nullptr;
     const int* types = de->tabs.ntypes > 1 ? d_types : nullptr;
     if (precision == TDMD_FP64) {
       de->fp64.reserve(static_cast<size_t>(natoms));
@@ -600,20 +608,21 @@ int32_t tdmd_device_eam_compute(tdmd_device_eam* de, const double* d_positions, 
       de->rec.reserve(static_cast<size_t>(natoms));
       const GeoD4F gf{de->rec.data(), img3(b)};
       launch_eam_density<GeoAoS64, double>(g, nl, natoms, de->tabs.d64, types, de->fp64.data(),
-                                           d_rho, d_fp, nullptr, ev, de->part.data(), lpa, s,
-                                           nullptr, de->rec.data());
+                                           d_rho, d_fp, nullptr, ev, part, lpa, s, nullptr,
+                                           de->rec.data());
       launch_eam_force<GeoD4F, true, double, double>(
           gf, nl, natoms, de->tabs.d64, types, de->fp64.data(), static_cast<double*>(d_forces), ev,
-          de->part.data() + static_cast<long long>(nblk) * kEvStride, lpa, s);
+          part_f, lpa, s);
     } else {
       TDMD_REQUIRE(precision == TDMD_MIXED, "unknown precision");
       de->fp32.reserve(static_cast<size_t>(natoms));
       const GeoAoS32 g = make_geo_aos32(d_positions, b);
       launch_eam(g, nl, natoms, de->tabs.d32, types, de->fp32.data(), d_rho, d_fp,
-                 static_cast<float*>(d_forces), ev, de->part.data(), lpa, s);
+                 static_cast<float*>(d_forces), ev, part, lpa, s);
     }
     if (ev) {
-      launch(k_reduce_partials, 1, reduce_threads(2 * nblk), 0, s, de->part.data(), 2 * nblk, d_energy, d_virial);
+      launch(k_reduce_partials, 1, reduce_threads(2 * nblk), 0, s, part, 2 * nblk, d_energy,
+             d_virial);
       TDMD_LAUNCH_CHECK();
     }
   });

@@ -255,3 +255,71 @@ def test_mixed_pair_interval(cuda, r):
     wf = (dphi + 2 * fp * drho)  # on atom 0, towards atom 1 when positive
     bound = 3e-6 * (abs(dphi) + abs(2 * fp * drho)) + 1e-7
     assert np.abs(f.cpu().numpy()[:, 0] - [wf, -wf]).max() <= bound
+
+
+# lanes per atom change between these sizes (8 at 40 000 atoms, 16 at 30 000 on
+# 148 SMs), so that the smaller system needs more block partials
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_device_eam_graphs_keep_their_scratch(cuda, precision):
+    """DeviceEam evaluations with energies, captured after a larger system was
+    evaluated, and replayed after a smaller one: the same bits as uncaptured."""
+    from tdmd_claude_b200 import Box, DeviceEam, DeviceNeighborList, EamAlloy
+    from tdmd_claude_b200 import workloads as W
+    t = W.cu_eam_tables()
+    de = DeviceEam()
+    de.upload_tables(EamAlloy.from_tables(t.ntypes, t.nrho, t.drho, t.nr, t.dr, t.cutoff, t.F,
+                                          t.rho, t.rphi))
+    a = 3.615
+
+    class Case:
+        def __init__(self, nz):
+            rng = np.random.default_rng(nz)
+            x = W.fcc_lattice(20, 25, nz, a)
+            hi = np.array([20, 25, nz]) * a
+            self.n, self.box = len(x), Box.make((0,) * 3, tuple(hi))
+            self.x = _dev(cuda, (x + rng.normal(0, 0.05, x.shape)) % hi)
+            self.types = cuda.ones(self.n, dtype=cuda.int32, device="cuda")
+            self.nl = DeviceNeighborList()
+            self.nl.build(self.x, self.n, self.box, t.cutoff, 0.3)
+            self.e, self.w = (cuda.zeros(k, dtype=cuda.float64, device="cuda") for k in (1, 6))
+            self.f = cuda.zeros((self.n, 3), device="cuda",
+                                dtype=cuda.float64 if precision == "fp64" else cuda.float32)
+            cuda.cuda.synchronize()
+
+        def run(self, prec=precision, stream=None, f=None):
+            de.compute(self.x, self.f if f is None else f, self.types, self.nl.d_neighbors(),
+                       self.nl.d_offsets(), self.nl.d_counts(), self.n, self.box, d_energy=self.e,
+                       d_virial=self.w, precision=prec, stream=stream)
+
+        def capture(self):
+            g = cuda.cuda.CUDAGraph()
+            with cuda.cuda.graph(g):
+                self.run(stream=cuda.cuda.current_stream())
+            return g
+
+        def out(self):
+            cuda.cuda.synchronize()
+            r = [x.cpu().numpy().copy() for x in (self.f, self.e, self.w)]
+            for x in (self.f, self.e, self.w):
+                x.zero_()
+            cuda.cuda.synchronize()
+            return r
+
+    big, small = Case(20), Case(15)
+    big.run()
+    want_big = big.out()
+    g_small = small.capture()  # nothing of this size ran before
+    small.out()
+    small.run()
+    want_small = small.out()
+    g_big = big.capture()
+    big.out()
+    small.run()
+    other = cuda.zeros((small.n, 3), device="cuda",
+                       dtype=cuda.float32 if precision == "fp64" else cuda.float64)
+    small.run(prec="mixed" if precision == "fp64" else "fp64", f=other)
+    small.out()
+    for case, g, want in ((big, g_big, want_big), (small, g_small, want_small)):
+        g.replay()
+        for got, w in zip(case.out(), want):
+            assert np.array_equal(got, w)
