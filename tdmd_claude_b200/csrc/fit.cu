@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "buffers.cuh"
@@ -88,6 +89,12 @@ __device__ __forceinline__ int pair_index(int ti, int tj, int nt) {
   return ti * nt - ti * (ti + 1) / 2 + tj;
 }
 
+unsigned high_word(double x) {
+  unsigned long long u;
+  std::memcpy(&u, &x, sizeof u);
+  return static_cast<unsigned>(u >> 32);
+}
+
 // Device view of the EAM coefficient arrays being fitted, the row copies the
 // passes read and the gradients (types 0-based here).
 struct FitEam {
@@ -98,14 +105,35 @@ struct FitEam {
   double* gphi;
   int nt, nsf, nsr;
   double drho, dr, inv_dr;
+  unsigned in_lo, in_span;
   __device__ __forceinline__ double4 rho_row(int t, int k) const {
     return ld_d4(rows + static_cast<long long>(t) * nsr + k);
   }
   __device__ __forceinline__ double4 phi_row(int p, int k) const {
     return ld_d4(rows + static_cast<long long>(nt + p) * nsr + k);
   }
+  // The interval int(r / dr) and the offset in it.  Each interval's
+  // coefficients are free parameters here: a pair on a knot must go where the
+  // division puts it, because the neighboring cubic may differ in value and
+  // slope and owns another part of the gradient.  So the product with 1/dr (as
+  // in spline_idx_mul) decides only offsets inside (in_lo, in_lo + in_span) of
+  // the high word; the others (about two in a million of thermal distances,
+  // whole shells of an ideal lattice, and what needs the clamp) take the
+  // quotient as the division rounds it: two Newton corrections of r * (1/dr)
+  // with exact remainders (Markstein's theorem).
   __device__ __forceinline__ int seg(double r, double& dx) const {
-    return spline_idx_mul(r, dr, inv_dr, nsr + 1, dx);
+    constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52
+    const double z = fma(r, inv_dr, -0.5) + kRound;
+    int k = __double2loint(z);
+    dx = fma(-(z - kRound), dr, r);
+    if (static_cast<unsigned>(__double2hiint(dx)) - in_lo >= in_span) {
+      double q = r * inv_dr;
+      q = fma(fma(-q, dr, r), inv_dr, q);
+      q = fma(fma(-q, dr, r), inv_dr, q);
+      k = min(static_cast<int>(q), nsr - 1);
+      dx = fma(-static_cast<double>(k), dr, r);
+    }
+    return k;
   }
 };
 
@@ -797,7 +825,14 @@ void Fit::eam(int ntypes, int nrho, double drho, int nr, double dr, const double
   const int npairs = ntypes * (ntypes + 1) / 2;
   const size_t nrows = static_cast<size_t>(ntypes + npairs) * (nr - 1);
   const CallScratch<double4> rows(rows_, nrows, nrows, s);
-  const FitEam e{F, rows.data(), gF, grho, gphi, ntypes, nrho - 1, nr - 1, drho, dr, 1.0 / dr};
+  // Offsets closer to a knot than the rounding of r / dr (r / dr < nr < 2^31:
+  // below 2^-21 dr), or than the cutoff may lie past the last knot, are not
+  // decided by the product with 1/dr.
+  const double edge = std::max(0x1p-20, 4e-12 * nr);
+  const unsigned in_lo = high_word(edge * dr) + 1;
+  const unsigned in_hi = high_word((1.0 - edge) * dr);  // offsets below it in the high word
+  const FitEam e{F,  rows.data(), gF,       grho,  gphi, ntypes, nrho - 1, nr - 1, drho,
+                 dr, 1.0 / dr,    in_lo, in_hi > in_lo ? in_hi - in_lo : 0};
   launch(k_fm_rows, std::min(2 * sm_count(), ceil_div(4ll * (ntypes + npairs) * (nr - 1), 256)),
          256, 0, s, rho, phi, ntypes, npairs, nr - 1, rows.data(), gF,
          4ll * (nrho - 1) * ntypes, grho, gphi);

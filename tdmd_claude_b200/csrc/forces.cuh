@@ -810,7 +810,8 @@ __device__ __forceinline__ int spline_idx(double r, double dr, int n, double& dx
 // round-to-nearest of q - 1/2 in the low word of q - 1/2 + 1.5 * 2^52, whose
 // difference from 1.5 * 2^52 is the interval as a double (no conversions).
 // Where q is within a rounding of a knot the neighboring interval may be
-// taken: value and derivative of the spline are continuous there, so the
+// taken (every other exact knot goes to the one below): only for splines whose
+// value and derivative are continuous, as build_spline's are, so that the
 // result changes by a rounding only.  0 <= q < 2^31.
 __device__ __forceinline__ int spline_idx_mul(double r, double dr, double inv_dr, int n,
                                               double& dx) {

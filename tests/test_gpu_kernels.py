@@ -323,3 +323,43 @@ def test_device_eam_graphs_keep_their_scratch(cuda, precision):
         g.replay()
         for got, w in zip(case.out(), want):
             assert np.array_equal(got, w)
+
+
+# the lattice constant and its double on an odd and an even knot, exactly
+# (dr = 1/256) or as the quotient rounds (dr = 0.005)
+@pytest.mark.parametrize("a,dr", [(513 / 256, 1 / 256), (2.005, 0.005), (3.615, 0.005)])
+@pytest.mark.parametrize("ntypes", [1, 3])
+def test_eam_fit_pairs_on_knots(cuda, oracle, a, dr, ntypes):
+    """Ideal simple-cubic snapshots (with vacancies, so that the densities
+    differ) whose shells sit on spline knots, with coefficients that jump there: loss and gradient belong to the interval
+    int(r / dr), as in the oracle (the bounds of the other FP64 fits)."""
+    from tdmd_claude_b200 import Box, EamAlloy
+    from tdmd_claude_b200 import workloads as W
+    from tdmd_claude_b200.fitting import ForceMatch, eam_coeff_tensors, eam_table_meta
+    rng = np.random.default_rng(ntypes)
+    kw = {} if ntypes == 1 else dict(beta_f=(4.8, 5.0, 5.2), A_phi=(0.55, 0.60, 0.65),
+                                     E_F=(1.1, 1.2, 1.3))
+    t = W.analytic_eam(nr=int(round(5.0 / dr)) + 1, **kw)
+    assert abs(t.dr - dr) < 1e-15
+    eam = EamAlloy.from_tables(t.ntypes, t.nrho, t.drho, t.nr, t.dr, t.cutoff, t.F, t.rho, t.rphi)
+    oe = oracle.OracleEam(t.ntypes, t.nrho, t.drho, t.nr, t.dr, t.cutoff, t.F, t.rho, t.rphi)
+    m = int(10.0 / a) + 1
+    x = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3) * a
+    pos = np.stack([rng.permutation(x)[:-9] for _ in range(2)])
+    types = rng.integers(1, ntypes + 1, size=pos.shape[:2]).astype(np.int32)
+    tgt = rng.normal(0.0, 0.3, size=pos.shape)
+    fm = ForceMatch(pos, types, Box.make((0,) * 3, (m * a,) * 3), t.cutoff, "fp64")
+    fm.set_targets(tgt)
+    F, rho, phi = eam_coeff_tensors(eam)
+    for kind, c in ((1, rho), (2, phi)):
+        c *= _dev(cuda, 1.0 + 0.1 * rng.normal(size=c.shape))
+        for k in range(len(c)):
+            oe.set_coeffs(kind, k, c[k].cpu().numpy())
+    loss = cuda.zeros(1, dtype=cuda.float64, device="cuda")
+    g = [cuda.empty_like(v) for v in (F, rho, phi)]
+    fm.eam(eam_table_meta(eam), F, rho, phi, loss, *g)
+    lo, *want = oe.fm_loss_grad(pos, types, (0,) * 3, (m * a,) * 3, tgt)
+    assert abs(loss.item() - lo) <= 1e-10 * lo
+    for got, ref in zip(g, want):
+        for sp in range(ref.shape[0]):
+            assert np.abs(got[sp].cpu().numpy() - ref[sp]).max() <= 1e-9 * np.abs(ref[sp]).max()
