@@ -137,10 +137,12 @@ struct FitEam {
   }
 };
 
-// 1/r as a double: the FP64 geometries' own, a division of the FP32 radius.
-__device__ __forceinline__ double inv_radius(double /*r*/, double rinv) { return rinv; }
-__device__ __forceinline__ double inv_radius(float r, float /*rinv*/) {
-  return 1.0 / static_cast<double>(r);
+// x / r, rounded once.
+__device__ __forceinline__ double over_radius(double x, double r, double rinv) {
+  return div_r(x, r, rinv);
+}
+__device__ __forceinline__ double over_radius(double x, float r, float /*rinv*/) {
+  return x / static_cast<double>(r);
 }
 
 // Block partial sums: lane merge -> warp -> block; thread 0 writes kPart.
@@ -256,9 +258,10 @@ __global__ void __launch_bounds__(kThreads) k_fm_morse_grad(Geo g, NbrView nl, i
         g.radius(o, pr, r, rinv, rd);
         const T ex = exp(-at * static_cast<T>(rd - r0));
         const T ome = T(1) - ex;
-        const double gd = (gi.x * static_cast<double>(pr.dx) + gi.y * static_cast<double>(pr.dy) +
-                           gi.z * static_cast<double>(pr.dz)) *
-                          inv_radius(r, rinv);
+        const double gd = over_radius(gi.x * static_cast<double>(pr.dx) +
+                                          gi.y * static_cast<double>(pr.dy) +
+                                          gi.z * static_cast<double>(pr.dz),
+                                      r, rinv);
         // df/dtheta * r (the 1/r is folded into gd)
         const T dD = -T(2) * at * ome * ex;
         const T da = -T(2) * Dt * (ome * ex - at * (T(1) - T(2) * ex) *
@@ -458,7 +461,7 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_weights(
         const double gd = (gi.x - gj.x) * static_cast<double>(pr.dx) +
                           (gi.y - gj.y) * static_cast<double>(pr.dy) +
                           (gi.z - gj.z) * static_cast<double>(pr.dz);
-        w -= dr * gd * inv_radius(r, rinv);
+        w -= over_radius(dr * gd, r, rinv);
       }
     }
   }
@@ -527,10 +530,10 @@ __global__ void __launch_bounds__(SHARED ? kPairThreads : kThreads) k_fm_eam_pai
       g.radius(o, pr, r, rinv, rd);
       double dx;
       const int kk = e.seg(rd, dx);
-      const double q = ((gi.x - gj.x) * static_cast<double>(pr.dx) +
-                        (gi.y - gj.y) * static_cast<double>(pr.dy) +
-                        (gi.z - gj.z) * static_cast<double>(pr.dz)) *
-                       inv_radius(r, rinv);
+      const double q = over_radius((gi.x - gj.x) * static_cast<double>(pr.dx) +
+                                       (gi.y - gj.y) * static_cast<double>(pr.dy) +
+                                       (gi.z - gj.z) * static_cast<double>(pr.dz),
+                                   r, rinv);
       if (SHARED && kk >= k0) {
         const double wd = -q * (gi.w + gj.w), wv = wi + wj;
         double* const s = sg + (kk - k0);

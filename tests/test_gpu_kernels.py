@@ -363,3 +363,30 @@ def test_eam_fit_pairs_on_knots(cuda, oracle, a, dr, ntypes):
     for got, ref in zip(g, want):
         for sp in range(ref.shape[0]):
             assert np.abs(got[sp].cpu().numpy() - ref[sp]).max() <= 1e-9 * np.abs(ref[sp]).max()
+
+
+def test_fit_divides_by_the_radius_once(cuda):
+    """Snapshots of two atoms, one pair to an interval, all coefficients zero:
+    the gradient of phi's b is a single quotient (G_i - G_j) . d / r, and
+    every one has the bits of the division."""
+    from tdmd_claude_b200 import Box
+    from tdmd_claude_b200.fitting import ForceMatch
+    rng = np.random.default_rng(12)
+    nsnap, nr, dr = 300, 2001, 0.0025
+    k = 5 * np.arange(nsnap) + 500
+    pos = np.full((nsnap, 2, 3), 6.0)
+    pos[:, 1, 0] += (k + rng.uniform(0.1, 0.9, nsnap)) * dr
+    tgt = rng.normal(size=pos.shape)
+    fm = ForceMatch(pos, np.ones((nsnap, 2), np.int32), Box.make((0,) * 3, (20.0,) * 3), 5.0,
+                    "fp64")
+    fm.set_targets(tgt)
+    z = [cuda.zeros((1, 4 * (nr - 1)), dtype=cuda.float64, device="cuda") for _ in range(3)]
+    g = [cuda.empty_like(v) for v in z]
+    loss = cuda.zeros(1, dtype=cuda.float64, device="cuda")
+    fm.eam(dict(ntypes=1, nrho=nr, drho=0.01, nr=nr, dr=dr), *z, loss, *g)
+    c = 1.0 / (3.0 * 2 * nsnap)
+    G = (2.0 * c) * (0.0 - tgt[:, :, 0])
+    d = pos[:, 0, 0] - pos[:, 1, 0]
+    want = np.zeros(nr - 1)
+    want[k] = -(((G[:, 0] - G[:, 1]) * d) / np.abs(d))
+    assert np.array_equal(g[2].cpu().numpy()[0, nr - 1:2 * (nr - 1)], want)
