@@ -282,6 +282,7 @@ void EamDevTables::upload(const tdmd_eam& e, cudaStream_t stream) {
   d32 = EamDev<float>{dtab32.data(), rtab32.data(), ftab.data(), nt, S, e.nr, e.nrho, dr32,
                       static_cast<float>(1.0 / e.dr), static_cast<float>(e.cutoff * e.cutoff),
                       e.drho, static_cast<float>(e.dr - static_cast<double>(dr32)), tbits};
+  d32.top = static_cast<unsigned>(std::min(e.nr - 2, (1 << 22) - 1));
 }
 
 // --------------------------------------------------------------------------

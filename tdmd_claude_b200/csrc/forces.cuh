@@ -786,6 +786,9 @@ struct EamDev {
   const double4* d4 = nullptr;
   const double2* d2 = nullptr;
   const double* da = nullptr;
+  // FP32 path: the last interval that spline_interval finds without a
+  // conversion, min(nr - 2, 2^22 - 1)
+  unsigned top = 0;
 };
 
 __device__ __forceinline__ int phi_slot(int ti, int tj, int nt) {
@@ -812,15 +815,17 @@ __device__ __forceinline__ int spline_idx(double r, double dr, int n, double& dx
 // Where q is within a rounding of a knot the neighboring interval may be
 // taken (every other exact knot goes to the one below): only for splines whose
 // value and derivative are continuous, as build_spline's are, so that the
-// result changes by a rounding only.  0 <= q < 2^31.
+// result changes by a rounding only.  From 2^32 on (a cutoff far beyond the
+// table) the sum leaves the low word, which its high word shows.
 __device__ __forceinline__ int spline_idx_mul(double r, double dr, double inv_dr, int n,
                                               double& dx) {
   constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52
   const double z = fma(r, inv_dr, -0.5) + kRound;
   int idx = __double2loint(z);
   dx = fma(-(z - kRound), dr, r);
-  if (static_cast<unsigned>(idx) > static_cast<unsigned>(n - 2)) {
-    idx = idx < 0 ? 0 : n - 2;
+  if (static_cast<unsigned>(idx) > static_cast<unsigned>(n - 2) ||
+      __double2hiint(z) != 0x43380000) {
+    idx = n - 2;
     dx = r - static_cast<double>(idx) * dr;
   }
   return idx;
@@ -828,14 +833,17 @@ __device__ __forceinline__ int spline_idx_mul(double r, double dr, double inv_dr
 
 // Interval of r in FP32 and the same number as a float, as spline_idx_mul has
 // it in FP64: no conversions, which run at a quarter of the rate of the
-// additions that replace them.  0 <= r / dr < 2^22.
+// additions that replace them.  From 2^22 on the sum with 1.5 * 2^23 is no
+// longer spaced by one, and beyond the table the last interval goes on: both
+// lie past e.top and take the conversion (r / dr is a whole float there, or the
+// interval is below 2^24: fi is exact).
 __device__ __forceinline__ int spline_interval(float r, const EamDev<float>& e, float& fi) {
   constexpr float kRound = 12582912.f;  // 1.5 * 2^23
   const float z = __fadd_rn(fmaf(r, e.inv_dr, -0.5f), kRound);
   int idx = __float_as_int(z) - 0x4B400000;
   fi = __fsub_rn(z, kRound);
-  if (static_cast<unsigned>(idx) > static_cast<unsigned>(e.nr - 2)) {
-    idx = idx < 0 ? 0 : e.nr - 2;
+  if (static_cast<unsigned>(idx) > e.top) {
+    idx = min(static_cast<int>(r * e.inv_dr), e.nr - 2);
     fi = static_cast<float>(idx);
   }
   return idx;

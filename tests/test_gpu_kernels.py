@@ -390,3 +390,54 @@ def test_fit_divides_by_the_radius_once(cuda):
     want = np.zeros(nr - 1)
     want[k] = -(((G[:, 0] - G[:, 1]) * d) / np.abs(d))
     assert np.array_equal(g[2].cpu().numpy()[0, nr - 1:2 * (nr - 1)], want)
+
+
+def _pair_eam(torch, eam, r, precision):
+    """(density, x force of atom 0) of two atoms r apart."""
+    from tdmd_claude_b200 import Box, DeviceEam
+    de = DeviceEam()
+    de.upload_tables(eam)
+    f = torch.zeros((2, 3), device="cuda",
+                    dtype=torch.float64 if precision == "fp64" else torch.float32)
+    rho = torch.zeros(2, dtype=torch.float64, device="cuda")
+    nbr, off, cnt = (_dev(torch, np.array(x, np.int32)) for x in ([1, 0], [0, 1], [1, 1]))
+    out = []
+    for x in r:
+        de.compute(_dev(torch, np.array([[0.0, 1.0, 2.0], [x, 1.0, 2.0]])), f,
+                   _dev(torch, np.ones(2, np.int32)), nbr.data_ptr(), off.data_ptr(),
+                   cnt.data_ptr(), 2, Box.make((-10.0,) * 3, (22.0,) * 3), d_rho=rho,
+                   precision=precision)
+        assert float(f[0, 0]) == -float(f[1, 0])
+        out.append((rho.cpu().numpy().copy(), float(f[0, 0])))
+    return out
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_eam_table_of_five_million_knots(cuda, precision):
+    """Distances on both sides of 2^22 = 4.19 M knots, where an FP32 sum with
+    1.5 * 2^23 stops being spaced by one: density and force of smooth
+    functions (FP32 distance, product and sum roundings: 1e-6 and 3e-6)."""
+    from tdmd_claude_b200 import EamAlloy
+    nr, dr = 5_000_001, 1e-6
+    x = np.arange(nr) * dr
+    F = -0.5 * np.arange(100) * 0.1  # F' = -1/2
+    eam = EamAlloy.from_tables(1, 100, 0.1, nr, dr, 5.0, F[None], np.exp(-x)[None],
+                               (x * np.exp(-2 * x))[None])
+    rs = [2.5, (2 ** 22 - 3) * dr, (2 ** 22 + 3.5) * dr, 4.5, 4.9]
+    for r, (rho, fx) in zip(rs, _pair_eam(cuda, eam, rs, precision)):
+        assert np.abs(rho / np.exp(-r) - 1).max() <= 1e-6
+        want = -2 * np.exp(-2 * r) + np.exp(-r)  # phi' + 2 F' rho', on atom 0 along +x
+        assert abs(fx - want) <= 3e-6 * np.exp(-r)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_eam_cutoff_far_beyond_the_table(cuda, precision):
+    """A table of ten knots that ends 2^32 spacings before the pair: the last
+    cubic goes on (exact straight lines here)."""
+    from tdmd_claude_b200 import EamAlloy
+    nr, dr = 10, 2.0 ** -33
+    k = np.arange(nr, dtype=float)
+    eam = EamAlloy.from_samples(1, nr, 1.0, nr, dr, 5.0, k[None], k[None], 3 * k[None])
+    for r, (rho, fx) in zip((2.5, 0.75), _pair_eam(cuda, eam, (2.5, 0.75), precision)):
+        assert np.allclose(rho, r / dr, rtol=1e-6)
+        assert np.allclose(fx, (3 + 2) / dr, rtol=1e-6)
