@@ -144,14 +144,16 @@ __global__ void k_sort_cells(const int* __restrict__ cell_start, const int* __re
 
 // The whole cell list of a small system in one block: histogram, scan,
 // scatter and per-cell sort with the counts in shared memory, instead of a
-// memset and four kernels of a few blocks each, whose time is launch latency.
-// Up to kOneBlockAtoms atoms (four per thread) and kOneBlockCells cells
-// (sixteen sorts per warp); beyond that one SM's share of the work nears the
-// launches it saves.  256 atoms: 758 -> 672 us per 100 steps; 2 767 atoms: 1.22
-// -> 1.18 ms.
+// memset and four kernels of a few blocks each, whose time is launch latency
+// (12.2-14.3 us a list in a replayed graph, whatever the size).  The block's
+// time grows with its atoms (about 1 us per 1024) and its cells (1.1 us per 32,
+// a sort per warp): 3.4 us at 256 atoms and 27 cells, 10.1 at 2767 and 140,
+// 10.9 at 3072 and 180.  The limits lie where both meet: 2767 atoms in 216
+// cells took 12.7 us in one block against 12.3, 2048 in 343 cells 15.7 against
+// 12.4, 4096 in 125 cells 19.1 against 14.3.
 constexpr int kOneBlockThreads = 1024;
-constexpr int kOneBlockAtoms = 4096;
-constexpr int kOneBlockCells = 512;
+constexpr int kOneBlockAtoms = 3072;  // three per thread
+constexpr int kOneBlockCells = 192;   // six sorts per warp
 template <class Load>
 __global__ void __launch_bounds__(kOneBlockThreads) k_cells_one_block(
     Load pos, int n, DevBox b, int ncells, int* __restrict__ atom_cell, int* cell_count,

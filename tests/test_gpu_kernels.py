@@ -170,12 +170,23 @@ def test_row_build_block_sizes(cuda, oracle, nc):
         assert np.array_equal(g, w)
 
 
-# the one-block rule's two limits (4096 atoms, 512 cells) and both sides of each
+# small systems, in one block or not, and cells of up to ~150 members
 @pytest.mark.parametrize("n,nc", [(1, (3, 3, 3)), (31, (3, 4, 5)), (4096, (8, 8, 8)),
                                   (4097, (8, 8, 8)), (4000, (9, 8, 8)), (4096, (3, 3, 3))])
 def test_cell_list_one_block(cuda, oracle, n, nc):
-    """Cell lists bit-exact around the one-block limits, with cells above 32
-    and above 128 members (27 cells of ~150 atoms)."""
+    """Cell lists bit-exact, with cells above 32 and above 128 members (27
+    cells of ~150 atoms)."""
+    _check_cell_list(cuda, oracle, n, nc)
+
+
+# the one-block rule's two limits (3072 atoms, 192 cells) and both sides of each
+@pytest.mark.parametrize("n,nc", [(3072, (4, 6, 8)), (3073, (4, 6, 8)), (3072, (5, 5, 8)),
+                                  (2, (4, 6, 8)), (3072, (3, 3, 3)), (1025, (3, 3, 21))])
+def test_cell_list_one_block_limits(cuda, oracle, n, nc):
+    _check_cell_list(cuda, oracle, n, nc)
+
+
+def _check_cell_list(cuda, oracle, n, nc):
     from tdmd_claude_b200 import Box, DeviceCellList
     rng = np.random.default_rng(n)
     hi = np.array(nc) * 5.0 + 0.1
