@@ -36,13 +36,17 @@ class DevArray {
 
   // Grow-only: keeps the allocation when it is already large enough.
   // Contents are NOT preserved on growth.
-  void reserve(size_t n) {
-    if (n <= cap_) return;
-    release();
-    void* p = nullptr;
-    TDMD_CU(cudaMalloc(&p, (n > 0 ? n : 1) * sizeof(T)));
-    p_ = static_cast<T*>(p);
-    cap_ = n;
+  void reserve(size_t n) { TDMD_CU(grow(n)); }
+  // The same, for an array that the caller can do without: false, with nothing
+  // held, where the device has no room for it.
+  bool try_reserve(size_t n) {
+    const cudaError_t e = grow(n);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      return false;
+    }
+    TDMD_CU(e);
+    return true;
   }
   void release() {
     if (p_) cudaFree(p_);
@@ -53,6 +57,16 @@ class DevArray {
   size_t capacity() const { return cap_; }
 
  private:
+  cudaError_t grow(size_t n) {
+    if (n <= cap_) return cudaSuccess;
+    release();
+    void* p = nullptr;
+    const cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+    if (e != cudaSuccess) return e;
+    p_ = static_cast<T*>(p);
+    cap_ = n;
+    return e;
+  }
   T* p_ = nullptr;
   size_t cap_ = 0;
 };

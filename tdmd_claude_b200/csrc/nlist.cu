@@ -999,8 +999,11 @@ int32_t tdmd_nlist_destroy(tdmd_nlist* nl) {
 // one sweep fills rows padded to a quarter above that, and a copy packs them
 // (118 661 atoms, 53 neighbors: count pass 75 us against 10 us for the copy).
 // A row that does not fit costs the second sweep again, from its exact
-// counts.  The padded rows are bounded at 2 GiB; larger lists keep the two
-// sweeps.
+// counts.  The padded rows are a convenience: they are bounded at 2 GiB and at
+// four times the last list plus 32 entries an atom (a crystal's take 1.7 times,
+// a gas's 2.1; beyond that a few long rows in a dense clump would size them for
+// every atom), and where the device has no room for them or beside them, the
+// build takes its two sweeps.
 int32_t tdmd_nlist_build(tdmd_nlist* nl, const double* d_positions, int64_t natoms,
                          const tdmd_box* box, double r_cut, double r_skin, void* stream) {
   return guarded([&] {
@@ -1010,6 +1013,8 @@ int32_t tdmd_nlist_build(tdmd_nlist* nl, const double* d_positions, int64_t nato
     TDMD_REQUIRE(natoms >= 0 && natoms < INT_MAX, "natoms out of range");
     TDMD_REQUIRE(natoms == 0 || d_positions, "positions are null");
     const long long last_max = nl->max_neighbors;
+    const double last_mean =
+        nl->natoms > 0 ? static_cast<double>(nl->total) / static_cast<double>(nl->natoms) : 0.0;
     nl->natoms = natoms;
     nl->total = 0;
     nl->max_neighbors = 0;
@@ -1024,8 +1029,10 @@ int32_t tdmd_nlist_build(tdmd_nlist* nl, const double* d_positions, int64_t nato
     nl->status.reserve(4);
     TDMD_CU(cudaMemsetAsync(nl->status.data(), 0, 4 * sizeof(int), s));
     const long long cap = last_max > 0 ? (last_max + last_max / 4 + 8 + 7) / 8 * 8ll : 0;
-    const bool one_pass = cap > 0 && cap * natoms <= (2ll << 30) / static_cast<long long>(sizeof(int));
-    if (one_pass) nl->rows.reserve(static_cast<size_t>(cap * natoms));
+    const bool one_pass =
+        cap > 0 && static_cast<double>(cap) <= 4.0 * last_mean + 32.0 &&
+        cap * natoms <= (2ll << 30) / static_cast<long long>(sizeof(int)) &&
+        nl->rows.try_reserve(static_cast<size_t>(cap * natoms));
     build_neighbor_rows(nl->cl, d_positions, PosLayout::AoS3, natoms, b, rl2,
                         one_pass ? nl->rows.data() : nullptr, nullptr,
                         one_pass ? static_cast<int>(cap) : 0, nl->counts.data(),
@@ -1037,8 +1044,14 @@ int32_t tdmd_nlist_build(tdmd_nlist* nl, const double* d_positions, int64_t nato
     TDMD_CU(cudaStreamSynchronize(s));
     nl->max_neighbors = h[1];
     nl->total = h[2];
-    nl->nbrs.reserve(static_cast<size_t>(nl->total > 0 ? nl->total : 1));
-    if (one_pass && !h[0]) {
+    const size_t want = static_cast<size_t>(nl->total > 0 ? nl->total : 1);
+    bool pack = one_pass && !h[0];
+    if (!nl->nbrs.try_reserve(want)) {
+      nl->rows.release();
+      pack = false;
+      nl->nbrs.reserve(want);
+    }
+    if (pack) {
       launch(k_pack_rows, ceil_div(natoms * kPackLanes, 256), 256, 0, s, nl->rows.data(),
              static_cast<int>(cap), nl->counts.data(), nl->offsets.data(),
              static_cast<int>(natoms), nl->nbrs.data());
