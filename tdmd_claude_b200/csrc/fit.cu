@@ -33,6 +33,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <optional>
 #include <vector>
 
 #include "buffers.cuh"
@@ -615,6 +616,11 @@ class Fit {
   template <class Fn>
   void with_geo(Fn&& fn) const;
   NbrView view() const { return NbrView{nbr_.data(), nullptr, cnt_.data(), cap_}; }
+  // doubles of the adjoint's block partials
+  size_t window_size() const {
+    return static_cast<size_t>(std::min(sm_count(), ceil_div(m_ * lpa_, kPairThreads))) * 7 *
+           kAdjointWindow;
+  }
 
   int nsnap_, n_;
   long long m_;
@@ -750,9 +756,11 @@ Fit::Fit(int nsnap, int natoms, const tdmd_box& box, const double* pos, const in
     build_neighbor_rows_batch(cl_, pos4_.data(), reps_.data(), cell_rep_.data(), rc_sq_,
                               nbr_.data(), cap_, cnt_.data(), nullptr, s);
     lpa_ = default_lpa(m_);
-    // the largest window a call can ask for, so that no call allocates it
-    window_.reserve(static_cast<size_t>(std::min(sm_count(), ceil_div(m_ * lpa_, kPairThreads))) *
-                    7 * kAdjointWindow);
+    // One element may take the shared-memory adjoint: its block partials, at
+    // the widest window a call can ask for, so that no call allocates them
+    // (0.75 ms of a first gradient).  Morse losses do without, so a device
+    // without room for them still gets its handle.
+    if (max_type_ == 1) window_.try_reserve(window_size());
     part_.reserve(2 * (static_cast<size_t>(force_blocks(m_, 32)) * kPart + kPart));
     TDMD_CU(cudaStreamSynchronize(s));
   } catch (...) {
@@ -847,6 +855,10 @@ void Fit::eam(int ntypes, int nrho, double drho, int nr, double dr, const double
   // The window of the shared-memory adjoint (one element).
   const int W = std::min(nr - 1, kAdjointWindow);
   const int grid = std::min(sm_count(), ceil_div(m_ * lpa_, kPairThreads));
+  std::optional<CallScratch<double>> window;
+  if (grad && ntypes == 1)
+    window.emplace(window_, window_size(), static_cast<size_t>(grid) * 7 * static_cast<size_t>(W),
+                   s);
   auto passes = [&](auto g, auto gf) {
     using Geo = decltype(g);
     using GeoF = decltype(gf);
@@ -864,8 +876,8 @@ void Fit::eam(int ntypes, int nrho, double drho, int nr, double dr, const double
           TDMD_CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem)));
           launch(kern, grid, kPairThreads, smem, s, g, nl, m, types_.data(), e, rc_sq_, G_.data(),
-                 wf_.data(), (nr - 1) - W, W, window_.data());
-          launch(k_fm_eam_window, ceil_div(7 * W, 32), 256, 0, s, window_.data(), grid, W,
+                 wf_.data(), (nr - 1) - W, W, window->data());
+          launch(k_fm_eam_window, ceil_div(7 * W, 32), 256, 0, s, window->data(), grid, W,
                  (nr - 1) - W, nr - 1, gphi, grho);
         } else {
           launch(k_fm_eam_pairs<Geo, L, false>, nblk, kThreads, 0, s, g, nl, m, types_.data(), e,

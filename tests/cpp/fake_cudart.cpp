@@ -2,6 +2,7 @@
 // running, so that a test can make them fail without a fault on the device.
 //   fake_fail(call, nth, code): the nth next run of `call` returns `code`.
 //   fake_runs(call): runs of `call` so far (failed ones included).
+//   fake_bytes(): bytes that cudaMalloc was asked for so far.
 #include <cuda_runtime_api.h>
 #include <dlfcn.h>
 
@@ -13,6 +14,7 @@ struct Call {
   long runs = 0, fail_in = 0;
   cudaError_t code = cudaSuccess;
 };
+long bytes = 0;
 Call calls[] = {{"cudaMalloc"}, {"cudaGraphInstantiate"}};
 
 void* real(const char* name) {
@@ -39,8 +41,10 @@ void fake_fail(const char* name, long nth, int code) {
   c->code = static_cast<cudaError_t>(code);
 }
 long fake_runs(const char* name) { return find(name)->runs; }
+long fake_bytes() { return bytes; }
 
 cudaError_t cudaMalloc(void** p, size_t n) {
+  bytes += static_cast<long>(n);
   if (fails(calls[0])) return calls[0].code;
   static const auto f = reinterpret_cast<cudaError_t (*)(void**, size_t)>(real("cudaMalloc"));
   return f(p, n);

@@ -1,6 +1,6 @@
 """Calls whose CUDA runtime call fails: an out-of-memory or an instantiation
 error code comes from a preloaded library (tests/cpp/fake_cudart.cpp) in place
-of the call, in a process of its own."""
+of the call, in a process of its own.  The same library counts allocations."""
 from __future__ import annotations
 
 import os
@@ -23,7 +23,7 @@ from oracle import oracle
 from tdmd_claude_b200 import *
 from tdmd_claude_b200 import workloads as W
 fake = C.CDLL(None)
-fake.fake_runs.restype = C.c_long
+fake.fake_runs.restype = fake.fake_bytes.restype = C.c_long
 def fail(call, nth, code):
     fake.fake_fail(call, C.c_long(nth), code)
 def runs(call=b"cudaMalloc"):
@@ -83,4 +83,55 @@ assert build(15 + 0.96 * (a - 15)) == 2   # the list: refused beside the rows, t
 assert build(a) == 1                 # the rows again
 build(clump)
 assert build(clump) == 0             # 300 neighbors an atom of the clump: two sweeps
+""")
+
+
+def test_fit_without_room_for_the_adjoint_window(child):
+    """The one-element adjoint's 10 MB of block partials: handles of several
+    elements never hold them, a handle that could not allocate them works and
+    asks again at the first gradient, and a captured first gradient has its
+    own in the graph."""
+    child("""
+from tdmd_claude_b200.fitting import ForceMatch, eam_coeff_tensors, eam_table_meta
+rng = np.random.default_rng(3)
+lat = W.fcc_lattice(4, 4, 4, 3.615)
+pos = np.stack([(lat + rng.normal(0, 0.1, lat.shape)) % (4 * 3.615) for _ in range(20)])
+tgt = rng.normal(0, 0.3, pos.shape)
+def make(types):
+    b, n = fake.fake_bytes(), runs()
+    fm = ForceMatch(pos, types, Box.make((0,) * 3, (4 * 3.615,) * 3), 5.0, "fp64")
+    fm.set_targets(tgt)
+    return fm, fake.fake_bytes() - b, runs() - n
+one = np.ones(pos.shape[:2], np.int32)
+_, bytes3, n3 = make(rng.integers(1, 4, pos.shape[:2]).astype(np.int32))
+fm, bytes1, n1 = make(one)
+assert n3 == n1 - 1 and bytes3 < bytes1 - 9e6
+t = W.cu_eam_tables()
+eam = EamAlloy.from_tables(t.ntypes, t.nrho, t.drho, t.nr, t.dr, t.cutoff, t.F, t.rho, t.rphi)
+meta, c = eam_table_meta(eam), eam_coeff_tensors(eam)
+loss, *g = [torch.empty_like(x) for x in (c[0][0, :1], *c)]
+def gradient(fm, allocations):
+    n = runs()
+    fm.eam(meta, *c, loss, *g)
+    assert runs() == n + allocations
+    return [x.cpu().numpy().copy() for x in (loss, *g)]
+def same(a, b):  # the adds' order is free: up to 1e4 terms an entry, some 100 times its size
+    for x, y in zip(a, b):
+        assert np.abs(x - y).max() <= 1e-10 * np.abs(y).max()
+want = gradient(fm, 1)               # the spline rows
+same(gradient(fm, 0), want)
+fail(b"cudaMalloc", n1 - 1, OOM)
+fm, _, n = make(one)
+assert n == n1
+same(gradient(fm, 2), want)          # the rows and the window
+fail(b"cudaMalloc", n1 - 1, OOM)
+fm = make(one)[0]
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    fm.eam(meta, *c, loss, *g)
+for x in (loss, *g):
+    x.fill_(7.0)
+graph.replay()
+torch.cuda.synchronize()
+same([x.cpu().numpy() for x in (loss, *g)], want)
 """)
