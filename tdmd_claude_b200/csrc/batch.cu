@@ -285,6 +285,9 @@ class Batch {
   void half_kick();
   void enqueue_step(const BatchStep& st);
   void run_segment(const std::vector<BatchStep>& seg, bool finalize, bool prologue);
+  void run_window(int target, bool flips);
+  void restore();
+  void abandon_window();
   void enqueue_prologue();
   void initial_forces();
   void grow_capacity(int max_count);
@@ -334,6 +337,7 @@ class Batch {
   DevArray<double4> pos4_alt_;
   DevArray<int4> q_alt_;
   bool in_alt_ = false;
+  bool window_open_ = false;  // the window's snapshot has been taken
   double4* pos4() const { return in_alt_ ? pos4_alt_.data() : pos4_.data(); }
   int4* q() const { return in_alt_ ? q_alt_.data() : q_.data(); }
   DevArray<double> vel_;
@@ -729,6 +733,7 @@ void Batch::run_segment(const std::vector<BatchStep>& seg, bool finalize, bool p
   };
   if (!cfg_.use_graphs) {
     if (prologue) enqueue_prologue();
+    window_open_ = window_open_ || prologue;
     for (const auto& st : seg) enqueue_step(st);
     close();
     return;
@@ -744,14 +749,12 @@ void Batch::run_segment(const std::vector<BatchStep>& seg, bool finalize, bool p
       graph_lru_.pop_back();
     }
     cudaGraph_t g = nullptr;
-    const bool start_in_alt = in_alt_;
     TDMD_CU(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     try {
       if (prologue) enqueue_prologue();
       for (const auto& st : seg) enqueue_step(st);
       close();
     } catch (...) {
-      in_alt_ = start_in_alt;
       cudaStreamEndCapture(stream_, &g);
       if (g) cudaGraphDestroy(g);
       throw;
@@ -770,6 +773,7 @@ void Batch::run_segment(const std::vector<BatchStep>& seg, bool finalize, bool p
     graph_lru_.push_front(key);
   }
   TDMD_CU(cudaGraphLaunch(it->second.first, stream_));
+  window_open_ = window_open_ || prologue;
   in_alt_ = end_in_alt;
   launches_ += it->second.second;
   ++graph_launches_;
@@ -858,6 +862,30 @@ void Batch::autotune(int* lanes2, int* batch2, double* ms24) {
   }
 }
 
+void Batch::restore() {
+  const size_t n = static_cast<size_t>(n_);
+  cudaStream_t s = stream_;
+  TDMD_CU(cudaMemcpyAsync(pos4_.data(), snap_pos4_.data(), n * sizeof(double4),
+                          cudaMemcpyDeviceToDevice, s));
+  TDMD_CU(cudaMemcpyAsync(vel_.data(), snap_vel_.data(), 3 * n * sizeof(double),
+                          cudaMemcpyDeviceToDevice, s));
+  if (mixed_)
+    TDMD_CU(cudaMemcpyAsync(q_.data(), snap_q_.data(), n * sizeof(int4),
+                            cudaMemcpyDeviceToDevice, s));
+}
+
+// As Scheduler::abandon_window: a failed window leaves its start.
+void Batch::abandon_window() {
+  in_alt_ = false;
+  if (!window_open_) return;
+  window_open_ = false;
+  initialized_ = false;
+  try {
+    restore();
+  } catch (...) {
+  }
+}
+
 void Batch::run_until(int target) {
   TDMD_REQUIRE(uploaded_, "run_until before upload");
   if (n_ == 0) {
@@ -871,8 +899,6 @@ void Batch::run_until(int target) {
     return;
   }
   const size_t n = static_cast<size_t>(n_);
-  cudaStream_t s = stream_;
-  const int step0 = step_, since0 = since_rebuild_;
   // snapshot buffers sized outside any stream capture
   snap_pos4_.reserve(n);
   snap_vel_.reserve(3 * n);
@@ -885,8 +911,19 @@ void Batch::run_until(int target) {
     pos4_alt_.reserve(n);
     if (mixed_) q_alt_.reserve(n);
   }
+  window_open_ = false;
+  try {
+    run_window(target, flips);
+  } catch (...) {
+    abandon_window();
+    throw;
+  }
+}
+
+void Batch::run_window(int target, bool flips) {
+  cudaStream_t s = stream_;
+  const int step0 = step_, since0 = since_rebuild_;
   for (int attempt = 0;; ++attempt) {
-    in_alt_ = false;
     TDMD_CU(cudaEventRecord(win_ev_[0], s));
     std::vector<BatchStep> plan;
     int since = since_rebuild_;
@@ -944,13 +981,7 @@ void Batch::run_until(int target) {
       throw Error{TDMD_ERR_NLIST_OVERFLOW, "neighbor list overflow persisted after retries"};
     ++retries_;
     grow_capacity(st[1]);
-    TDMD_CU(cudaMemcpyAsync(pos4_.data(), snap_pos4_.data(), n * sizeof(double4),
-                            cudaMemcpyDeviceToDevice, s));
-    TDMD_CU(cudaMemcpyAsync(vel_.data(), snap_vel_.data(), 3 * n * sizeof(double),
-                            cudaMemcpyDeviceToDevice, s));
-    if (mixed_)
-      TDMD_CU(cudaMemcpyAsync(q_.data(), snap_q_.data(), n * sizeof(int4),
-                              cudaMemcpyDeviceToDevice, s));
+    restore();
     step_ = step0;
     since_rebuild_ = since0;
     // Rebuild into the new capacity and recompute the forces of the

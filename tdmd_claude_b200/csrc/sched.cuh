@@ -164,6 +164,8 @@ class Scheduler {
   std::vector<StepPlan> plan_steps(int target, int* since_out) const;
   void reserve_snapshot();
   void restore();
+  void run_window(int target);
+  void abandon_window();
   void clear_graphs();
   void prof_begin(int cat);
   void prof_end(int cat);
@@ -212,6 +214,7 @@ class Scheduler {
   DevArray<float> f32_alt_;
   DevArray<int> types_alt_, ids_alt_;
   bool in_alt_ = false;  // inside a window: the positions are in the second buffers
+  bool window_open_ = false;  // the window's snapshot has been taken
   bool cells_from_upload_ = false;  // cl_ holds the cells of the reordered upload
   DevArray<double> masses_;
   DevArray<double> inv_mm_;  // 1 / (m mvv2e) per type: the kick factor per unit dt

@@ -1054,6 +1054,7 @@ void Scheduler::run_segment(const std::vector<StepPlan>& seg, bool finalize, int
   const long long l0 = launches_;
   if (!cfg_.use_graphs) {
     enqueue_prologue(prologue);
+    if (prologue & kPrologueSnapshot) window_open_ = true;
     for (const auto& st : seg) enqueue_step(st);
     if (finalize) enqueue_finalize();
     return;
@@ -1077,14 +1078,12 @@ void Scheduler::run_segment(const std::vector<StepPlan>& seg, bool finalize, int
       prof_sink_ = &ge.prof;
       suppress_programmatic_launch(true);
     }
-    const bool start_in_alt = in_alt_;
     TDMD_CU(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     try {
       enqueue_prologue(prologue);
       for (const auto& st : seg) enqueue_step(st);
       if (finalize) enqueue_finalize();
     } catch (...) {
-      in_alt_ = start_in_alt;
       prof_sink_ = nullptr;
       suppress_programmatic_launch(false);
       cudaStreamEndCapture(stream_, &g);
@@ -1107,6 +1106,7 @@ void Scheduler::run_segment(const std::vector<StepPlan>& seg, bool finalize, int
     graph_lru_.push_front(key);
   }
   TDMD_CU(cudaGraphLaunch(it->second.exec, stream_));
+  if (prologue & kPrologueSnapshot) window_open_ = true;
   in_alt_ = end_in_alt;
   launches_ += it->second.kernels;
   ++graph_launches_;
@@ -1222,6 +1222,20 @@ void Scheduler::restore() {
                           cudaMemcpyDeviceToDevice, s));
 }
 
+// A window that failed (a CUDA call's error, rows that keep overflowing): the
+// state is the window's start again, in the first position buffers, and the
+// next use builds its list and forces anew.
+void Scheduler::abandon_window() {
+  in_alt_ = false;
+  if (!window_open_) return;
+  window_open_ = false;
+  initialized_ = false;
+  try {
+    restore();
+  } catch (...) {  // the device itself failed: the first error is the one to report
+  }
+}
+
 void Scheduler::run_until(int target) {
   TDMD_REQUIRE(uploaded_, "run_until before upload");
   if (n_ == 0) {
@@ -1238,10 +1252,19 @@ void Scheduler::run_until(int target) {
     TDMD_CU(cudaStreamSynchronize(stream_));
     return;
   }
-  const int step0 = step_, since0 = since_rebuild_;
   reserve_snapshot();
+  window_open_ = false;
+  try {
+    run_window(target);
+  } catch (...) {
+    abandon_window();
+    throw;
+  }
+}
+
+void Scheduler::run_window(int target) {
+  const int step0 = step_, since0 = since_rebuild_;
   for (int attempt = 0;; ++attempt) {
-    in_alt_ = false;
     TDMD_CU(cudaEventRecord(win_ev_[0], stream_));
     // The snapshot and the flag reset go into the first segment's graph: one
     // submission per window.  A pending first-list overflow flag stays set

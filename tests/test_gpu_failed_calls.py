@@ -135,3 +135,61 @@ graph.replay()
 torch.cuda.synchronize()
 same([x.cpu().numpy() for x in (loss, *g)], want)
 """)
+
+
+def test_failed_window_leaves_its_start(child):
+    """A graph that cannot be instantiated in the middle of a window: the error
+    is reported, the state is the window's start, the next window runs from
+    there, and a new upload has nothing of the old one."""
+    child("""
+s = W.fcc_system(4, 3.615, 600.0, 3)
+t = W.cu_eam_tables()
+eam = EamAlloy.from_tables(t.ntypes, t.nrho, t.drho, t.nr, t.dr, t.cutoff, t.F, t.rho, t.rphi)
+L = np.array(s.hi) - np.array(s.lo)
+moved = (s.positions + np.random.default_rng(1).normal(0, 0.1, s.positions.shape) - s.lo) % L + s.lo
+def make(pot, precision, batch):
+    cfg = make_config(r_skin=0.5, rebuild_every=6, precision=precision, lanes_per_atom=8)
+    p = MorseParams.make(*W.MORSE_CU) if pot == "morse" else eam
+    return (ReplicaBatch([Box.make(s.lo, s.hi)], [s.n], p, cfg) if batch else
+            FastPipelineScheduler(Box.make(s.lo, s.hi), s.n, p, cfg))
+def up(m, x, batch):
+    if batch:
+        m.upload(x, s.velocities, s.types, s.masses)
+    else:
+        m.upload(x, s.velocities, None, s.types, s.ids, s.masses)
+def state(m, batch):
+    d = m.download()
+    return [np.array(v) for v in (d if batch else (d.positions, d.velocities, d.forces))]
+for pot in ("morse", "eam"):
+    for precision in ("fp64", "mixed"):
+        for batch in (False, True):
+            for end in (30, 31):      # an odd and an even number of fused drifts
+                m, good = make(pot, precision, batch), make(pot, precision, batch)
+                up(m, s.positions, batch), up(good, s.positions, batch)
+                m.run_until(5), good.run_until(5)
+                start = state(good, batch)
+                fail(b"cudaGraphInstantiate", 2, OOM)
+                try:
+                    m.run_until(end)
+                    raise SystemExit("no error")
+                except TdmdError as e:
+                    assert "OUT_OF_MEMORY" in str(e), e
+                for a, b in zip(state(m, batch)[:2], start):
+                    assert np.array_equal(a, b), (pot, precision, batch)
+                m.run_until(end), good.run_until(end)   # (the lists' steps differ)
+                tol = 1e-9 if precision == "fp64" else 1e-4
+                d = state(m, batch)[0] - state(good, batch)[0]
+                assert np.abs(d - np.round(d / L) * L).max() <= tol
+                fail(b"cudaGraphInstantiate", 2, OOM)
+                try:
+                    m.run_until(end + 26)
+                    raise SystemExit("no error")
+                except TdmdError:
+                    pass
+                new = make(pot, precision, batch)
+                for x in (m, new):
+                    up(x, moved, batch)
+                    x.run_until(1)
+                for a, b in zip(state(m, batch), state(new, batch)):
+                    assert np.array_equal(a, b), (pot, precision, batch)
+""")
