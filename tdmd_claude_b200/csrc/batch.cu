@@ -905,12 +905,10 @@ void Batch::run_until(int target) {
   if (mixed_) snap_q_.reserve(n);
   // Morse graph windows: the force passes carry the next step's kick + drift
   // into second position buffers (EAM passes read gather records and update
-  // in place), as in the single-system scheduler.
-  const bool flips = !eam_ && cfg_.use_graphs != 0;
-  if (flips) {
-    pos4_alt_.reserve(n);
-    if (mixed_) q_alt_.reserve(n);
-  }
+  // in place), as in the single-system scheduler.  Without room for them the
+  // drift stays a launch of its own (same bits).
+  const bool flips = !eam_ && cfg_.use_graphs != 0 && pos4_alt_.try_reserve(n) &&
+                     (!mixed_ || q_alt_.try_reserve(n));
   window_open_ = false;
   try {
     run_window(target, flips);

@@ -193,3 +193,29 @@ for pot in ("morse", "eam"):
                 for a, b in zip(state(m, batch), state(new, batch)):
                     assert np.array_equal(a, b), (pot, precision, batch)
 """)
+
+
+def test_batch_without_room_for_second_positions(child):
+    """A Morse batch whose second position buffers cannot be allocated drifts
+    in launches of its own: the same bits."""
+    child("""
+s = W.fcc_system(4, 3.615, 600.0, 3)
+# a first window allocates its snapshot (2 arrays, 3 in mixed), then these (1, 2)
+for precision, refused in (("fp64", 3), ("mixed", 4), ("mixed", 5)):
+    out = []
+    for nth in (0, refused):
+        cfg = make_config(r_skin=0.5, rebuild_every=6, precision=precision, lanes_per_atom=8)
+        m = ReplicaBatch([Box.make(s.lo, s.hi)], [s.n], MorseParams.make(*W.MORSE_CU), cfg)
+        m.upload(s.positions, s.velocities, s.types, s.masses)
+        m.run_until(0)
+        n = runs()
+        fail(b"cudaMalloc", nth, OOM)
+        m.run_until(8)
+        assert not nth or runs() - n == nth
+        for t in (8, 17, 40):
+            m.run_until(t)
+            out.append([np.array(v) for v in m.download()])
+    for a, b in zip(out[:3], out[3:]):
+        for x, y in zip(a, b):
+            assert np.array_equal(x, y)
+""")
