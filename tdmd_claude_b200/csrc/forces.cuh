@@ -212,10 +212,12 @@ __device__ __forceinline__ void radius_d(double x, double& r, double& rinv) {
 }
 
 // x / r: FP64 corrects the product with 1/r by its exact remainder (the
-// division's rounding); FP32 multiplies by rsqrt.
+// division's rounding; an infinite quotient has no remainder and stays, as the
+// division leaves it); FP32 multiplies by rsqrt.
 __device__ __forceinline__ double div_r(double x, double r, double rinv) {
   const double q = x * rinv;
-  return fma(fma(-q, r, x), rinv, q);
+  const double c = fma(fma(-q, r, x), rinv, q);
+  return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : c;
 }
 __device__ __forceinline__ float div_r(float x, float /*r*/, float rinv) { return x * rinv; }
 

@@ -452,3 +452,19 @@ def test_eam_cutoff_far_beyond_the_table(cuda, precision):
     for r, (rho, fx) in zip((2.5, 0.75), _pair_eam(cuda, eam, (2.5, 0.75), precision)):
         assert np.allclose(rho, r / dr, rtol=1e-6)
         assert np.allclose(fx, (3 + 2) / dr, rtol=1e-6)
+
+
+# a Morse force whose two exponentials overflow together, and two atoms so close
+# that r^2 underflows
+@pytest.mark.parametrize("alpha,d", [(400.0, (1.1, -1.2, 1.3)), (1.4, (1e-170, -1e-171, 1e-170))])
+def test_infinite_forces_keep_their_sign(cuda, alpha, d):
+    """FP64 pair forces beyond the range are infinities of the sign that the
+    division gives, not NaN."""
+    from tdmd_claude_b200 import Box, MorseParams, compute_morse_gpu
+    pos = np.array([[0.0, 0.0, 0.0], d])
+    f = cuda.zeros((2, 3), dtype=cuda.float64, device="cuda")
+    nbr, off, cnt = (_dev(cuda, np.array(x, np.int32)) for x in ([1, 0], [0, 1], [1, 1]))
+    compute_morse_gpu(_dev(cuda, pos), f, nbr.data_ptr(), off.data_ptr(), cnt.data_ptr(), 2,
+                      Box.make((-10.0,) * 3, (10.0,) * 3), MorseParams.make(0.3, alpha, 3.0, 5.0))
+    want = np.sign(pos[0] - pos[1]) * np.inf  # repulsive
+    assert np.array_equal(f.cpu().numpy(), [want, -want])
