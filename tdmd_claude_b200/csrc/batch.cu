@@ -583,7 +583,7 @@ void Batch::force(bool kd, bool pea, int parts) {
   const int n = static_cast<int>(n_);
   const Tune td{lpa_d_, nu_d_}, tf{lpa_, nu_};
   const bool dens = parts & kPassDensity, pair = parts & kPassForce;
-    if (eam_) {
+  if (eam_) {
     // Density + embedding, then forces, over all replicas at once (the
     // single scheduler's passes on the batched geometries).
     const int* types = eam_->ntypes > 1 ? types_.data() : nullptr;

@@ -409,7 +409,8 @@ __global__ void __launch_bounds__(kThreads) k_fm_eam_force(
         const T dphi = row_deriv<T>(e.phi_row(multi ? pair_index(ti, tj, e.nt) : 0, kk), dx);
         const T drj = row_deriv<T>(e.rho_row(tj, kk), dx);
         const T dri = ti == tj ? drj : row_deriv<T>(e.rho_row(ti, kk), dx);
-        const T fpair = -div_r(dphi + fpi * drj + static_cast<T>(g.gather_fp(pr, 0)) * dri, r, rinv);
+        const T fpj = static_cast<T>(g.gather_fp(pr, 0));
+        const T fpair = -div_r(dphi + fpi * drj + fpj * dri, r, rinv);
         fx.add(mul_rn(fpair, pr.dx));
         fy.add(mul_rn(fpair, pr.dy));
         fz.add(mul_rn(fpair, pr.dz));

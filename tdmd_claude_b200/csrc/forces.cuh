@@ -16,11 +16,10 @@
 //    delta cast to FP32), or fixed-point int32 positions whose wrapped
 //    difference IS the minimum image (scheduler's mixed path, 16-byte
 //    gathers).
-//  * Mixed precision: FP32 distances/splines/forces with rsqrt-based 1/r,
-//    a refined radius (two floats for the spline offset, FP64 for the Morse
-//    exponent),
-//    compensated FP32 per-atom sums (Kahan per lane, TwoSum across lanes);
-//    energies and virial always accumulate in FP64.
+//  * Mixed precision: FP32 distances/splines/forces with rsqrt-based 1/r, a
+//    refined radius (two floats for the spline offset, FP64 for the Morse
+//    exponent), compensated FP32 per-atom sums (Kahan per lane, TwoSum across
+//    lanes); energies and virial always accumulate in FP64.
 //  * Energy/virial (template EV): per-block FP64 partials reduced later in a
 //    fixed order by k_reduce_partials.
 //  * EAM splines: the density pass reads rows (a,b,c,d) of rho_t; the force
@@ -211,6 +210,13 @@ __device__ __forceinline__ void radius_d(double x, double& r, double& rinv) {
   }
 }
 
+// |r_i - r_j| alone.
+__device__ __forceinline__ double root_d(double x) {
+  double r, rinv;
+  radius_d(x, r, rinv);
+  return r;
+}
+
 // x / r: FP64 corrects the product with 1/r by its exact remainder (the
 // division's rounding; an infinite quotient has no remainder and stays, as the
 // division leaves it); FP32 multiplies by rsqrt.
@@ -235,9 +241,6 @@ struct PairQ {
   int w;  // the neighbor's 4th word
 };
 
-// |r| and 1/|r| in FP32 and the FP64-refined radius from a PairQ: with
-// r = sqrt(r2) in FP32, r2d - r*r = res + (r2 - r*r), the second term exact
-// by FMA; one Newton step rd = r + (r2d - r*r) / (2r).
 // 1/sqrt of a fixed-point pair's r^2: zero or at least (L/2^32)^2, so the
 // reciprocal root needs none of rsqrtf's rescaling of subnormals (two
 // predicated multiplications and a compare a pair; same bits).
@@ -263,6 +266,9 @@ __device__ __forceinline__ float q_residual(int ix, int iy, int iz, int iso, dou
   return static_cast<float>(x * x * s2x + y * y * s2y + z * z * s2z - static_cast<double>(r2));
 }
 
+// |r| and 1/|r| in FP32 and the FP64-refined radius from a PairQ: with
+// r = sqrt(r2) in FP32, r2d - r*r = res + (r2 - r*r), the second term exact
+// by FMA; one Newton step rd = r + (r2d - r*r) / (2r).
 __device__ __forceinline__ void radius_q(float r2, float res, float& r, float& rinv, double& rd) {
   rinv = rsqrt_q(r2);
   r = r2 * rinv;
@@ -328,11 +334,7 @@ struct GeoD4 {  // FP64, scheduler layout double4 {x,y,z,type}
     radius_d(pr.r2, r, rinv);
     corr = 0.0;
   }
-  __device__ __forceinline__ T radius_fast(const Pair& pr) const {
-    T r, rinv;
-    radius_d(pr.r2, r, rinv);
-    return r;
-  }
+  __device__ __forceinline__ T radius_fast(const Pair& pr) const { return root_d(pr.r2); }
 };
 
 // FP64 pair from a gather record: the neighbor's F'(rho) rides along.
@@ -363,20 +365,10 @@ struct GeoD4F {
     pr.r2 = pr.dx * pr.dx + pr.dy * pr.dy + pr.dz * pr.dz;
     pr.fw = q.w;
   }
-  __device__ __forceinline__ void radius(const Own&, const Pair& pr, T& r, T& rinv,
-                                         double& rd) const {
-    radius_d(pr.r2, r, rinv);
-    rd = r;
-  }
   __device__ __forceinline__ void radius2(const Own&, const Pair& pr, T& r, T& rinv,
                                           T& corr) const {
     radius_d(pr.r2, r, rinv);
     corr = 0.0;
-  }
-  __device__ __forceinline__ T radius_fast(const Pair& pr) const {
-    T r, rinv;
-    radius_d(pr.r2, r, rinv);
-    return r;
   }
   // F'(rho_j) of a pair's record
   __device__ __forceinline__ double gather_fp(const Pair& pr, int /*tmask*/) const {
@@ -414,11 +406,7 @@ struct GeoAoS64 {  // FP64, reference Vec3D AoS
     radius_d(pr.r2, r, rinv);
     corr = 0.0;
   }
-  __device__ __forceinline__ T radius_fast(const Pair& pr) const {
-    T r, rinv;
-    radius_d(pr.r2, r, rinv);
-    return r;
-  }
+  __device__ __forceinline__ T radius_fast(const Pair& pr) const { return root_d(pr.r2); }
 };
 
 // Mixed on the reference layout (free functions): the delta is formed in
@@ -552,7 +540,6 @@ struct Acc<float> {
 __device__ __forceinline__ double mul_rn(double a, double b) { return a * b; }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 
-
 // Force output: AoS float3 or double3.
 template <class F>
 struct ForceOut {
@@ -655,8 +642,9 @@ __device__ __forceinline__ void kick_drift_atom(const KickDrift& k, int i, FT fx
   k.v[3ll * i + 2] = vz;
   (ALT ? k.pos4_alt : k.pos4)[i] = p;
   if constexpr (sizeof(FT) == sizeof(float))
-    (ALT ? k.q_alt : k.q)[i] = make_int4(encode_q(p.x, b.qlo[0], b.qinv[0]), encode_q(p.y, b.qlo[1], b.qinv[1]),
-                       encode_q(p.z, b.qlo[2], b.qinv[2]), t);
+    (ALT ? k.q_alt : k.q)[i] =
+        make_int4(encode_q(p.x, b.qlo[0], b.qinv[0]), encode_q(p.y, b.qlo[1], b.qinv[1]),
+                  encode_q(p.z, b.qlo[2], b.qinv[2]), t);
 }
 
 // --------------------------------------------------------------------------
@@ -853,11 +841,12 @@ __device__ __forceinline__ int spline_interval(float r, const EamDev<float>& e, 
 
 // Interval from r, offset from the refined radius r + corr (FP32: the knot
 // spacing as dr + dr_lo, so that the offset rounds at its own size, below
-// 2e-10 A).  Without the FP64 radius, whose four conversions and two FP64
-// operations a pair sat in the chain from distance to spline row, and with the
-// intervals above: mixed EAM 131k 3.84 -> 3.81 ms per 50 steps, 1.05 M atoms
-// 11.81 -> 11.59 ms per 20, ternary 55k NVT 3.06 -> 2.97 ms per 50; 2 767 atoms
-// within the spread of its launch shapes (1.14-1.19 ms).
+// 2e-10 A; force, energy and density errors against FP64 are those of an FP64
+// offset to four digits, 500 to 10 000 knots).  Without the FP64 radius, whose
+// four conversions and two FP64 operations a pair sat in the chain from
+// distance to spline row, and with the intervals above: mixed EAM 131k 3.87 ->
+// 3.82 ms per 50 steps, 1.05 M atoms 11.89 -> 11.73 ms per 20; ternary 55k NVT
+// and 2 767 atoms within their spread.
 __device__ __forceinline__ int spline_at(double r, double /*corr*/, const EamDev<double>& e,
                                          double& sx) {
   return spline_idx_mul(r, e.dr, e.inv_dr, e.nr, sx);

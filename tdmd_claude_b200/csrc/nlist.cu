@@ -250,10 +250,10 @@ bool one_block_cells(long long n, long long ncells) {
 constexpr int kRowThreads = 128;
 // One system of few cells (at most two per SM) gets CTAs of 512 threads: with
 // the chip idle, the time is one cell's serial chain -- staging, then the rows
-// a warp takes in turn -- and more warps shorten it.  Above that the smaller
-// CTAs fill the SMs better (131k, 9 261 cells: 64 and 128 threads compared).
-// 256 atoms, 27 cells: 808 -> 758 us per 100 steps; 2 767 atoms, 140 cells:
-// 1.31 -> 1.22 ms.
+// a warp takes in turn -- and more warps shorten it.  List builds at 294 cells,
+// 128 against 512 threads: 16 atoms a cell 61 and 51 us, 20: 67 and 61, 30: 86
+// and 66, 8: no difference.  For thousands of cells the smaller CTAs fill the
+// SMs better.
 constexpr int kRowThreadsFew = 512;
 constexpr int kStageCap = 1536;  // staged candidate records (24 KiB)
 constexpr int kSlabMax = 128;    // center atoms handled as warp slabs
@@ -283,9 +283,9 @@ template <int RT>
 struct RowSmem {
   int s_start[27], s_pre[28];
   int s_max[RT / 32];
-  int s_wcnt[RT / 32];  // kept candidates per warp (staging chunk)
-  float s_bb[6];                 // center cell's bounding box: min xyz, max xyz
-  int s_c0;                      // staged index of the center cell's first atom
+  int s_wcnt[RT / 32];      // kept candidates per warp (staging chunk)
+  float s_bb[6];            // center cell's bounding box: min xyz, max xyz
+  int s_c0;                 // staged index of the center cell's first atom
 };
 
 // Shared memory of the warp-slab variant (4.3 KiB more per CTA).
@@ -656,9 +656,9 @@ __global__ void __launch_bounds__(RT) k_build_cells(
   // launch from the mean cell occupancy, so that more CTAs fit on an SM).
   extern __shared__ float4 stage[];
   __shared__ RowSmem<RT> sm;
-  build_cell_rows<RT, Load, WRAP, WRITE, false>(sm, stage, stage_cap, nullptr, pos, b, blockIdx.x,
-                                            cell_start, cell_count, cell_atoms, rl2, lo_f, hi_f,
-                                            nbr, row_off, cap, counts, status, report_max != 0);
+  build_cell_rows<RT, Load, WRAP, WRITE, false>(
+      sm, stage, stage_cap, nullptr, pos, b, blockIdx.x, cell_start, cell_count, cell_atoms, rl2,
+      lo_f, hi_f, nbr, row_off, cap, counts, status, report_max != 0);
 }
 
 // Batched replicas: one CTA per cell of any replica (cells of replica r are
@@ -679,16 +679,15 @@ __global__ void __launch_bounds__(kRowThreads) k_build_cells_batch(
   if (threadIdx.x == 0) d = reps[__ldg(cell_rep + gc)];
   __syncthreads();
   if (d.wrap)
-    build_cell_rows<kRowThreads, LoadD4, true, WRITE, true>(sm, stage, kStageCap, &ss, pos, d.box, gc - d.cell0,
-                                               cell_start + d.cell0, cell_count + d.cell0,
-                                               cell_atoms, rl2, d.lo_f, d.hi_f, nbr, nullptr,
-                                               cap, counts, status, false);
+    build_cell_rows<kRowThreads, LoadD4, true, WRITE, true>(
+        sm, stage, kStageCap, &ss, pos, d.box, gc - d.cell0, cell_start + d.cell0,
+        cell_count + d.cell0, cell_atoms, rl2, d.lo_f, d.hi_f, nbr, nullptr, cap, counts, status,
+        false);
   else
-    build_cell_rows<kRowThreads, LoadD4, false, WRITE, true>(sm, stage, kStageCap, &ss, pos, d.box,
-                                                gc - d.cell0,
-                                                cell_start + d.cell0, cell_count + d.cell0,
-                                                cell_atoms, rl2, d.lo_f, d.hi_f, nbr, nullptr,
-                                                cap, counts, status, false);
+    build_cell_rows<kRowThreads, LoadD4, false, WRITE, true>(
+        sm, stage, kStageCap, &ss, pos, d.box, gc - d.cell0, cell_start + d.cell0,
+        cell_count + d.cell0, cell_atoms, rl2, d.lo_f, d.hi_f, nbr, nullptr, cap, counts, status,
+        false);
 }
 
 // Batched binning: the replica of atom i is rep[i]; its cell is the

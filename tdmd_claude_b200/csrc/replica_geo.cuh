@@ -115,11 +115,7 @@ struct GeoD4B {
     radius_d(pr.r2, r, rinv);
     corr = 0.0;
   }
-  __device__ __forceinline__ T radius_fast(const Pair& pr) const {
-    T r, rinv;
-    radius_d(pr.r2, r, rinv);
-    return r;
-  }
+  __device__ __forceinline__ T radius_fast(const Pair& pr) const { return root_d(pr.r2); }
 };
 
 // FP64 gather records {x, y, z, F'(rho)} of a batch (written by the
@@ -153,11 +149,6 @@ struct GeoD4BF {
                                           T& corr) const {
     radius_d(pr.r2, r, rinv);
     corr = 0.0;
-  }
-  __device__ __forceinline__ T radius_fast(const Pair& pr) const {
-    T r, rinv;
-    radius_d(pr.r2, r, rinv);
-    return r;
   }
   __device__ __forceinline__ double gather_fp(const Pair& pr, int /*tmask*/) const {
     return pr.fw;

@@ -882,7 +882,8 @@ void Scheduler::enqueue_force(bool ev, bool kd, int parts) {
     TDMD_REQUIRE(parts == kPassBoth, "energy/virial needs both passes");
     const int nrec = kind_ == TDMD_POT_EAM ? nblk_d + nblk : nblk;
     TDMD_CU(cudaMemsetAsync(ctl_ev(), 0, sizeof(double) * 7, s));
-    launch(k_reduce_partials, 1, reduce_threads(nrec), 0, s, ev_part_.data(), nrec, ctl_ev(), ctl_ev() + 1);
+    launch(k_reduce_partials, 1, reduce_threads(nrec), 0, s, ev_part_.data(), nrec, ctl_ev(),
+           ctl_ev() + 1);
     TDMD_LAUNCH_CHECK();
     launches_ += 1;
   }
