@@ -468,3 +468,39 @@ def test_infinite_forces_keep_their_sign(cuda, alpha, d):
                       Box.make((-10.0,) * 3, (10.0,) * 3), MorseParams.make(0.3, alpha, 3.0, 5.0))
     want = np.sign(pos[0] - pos[1]) * np.inf  # repulsive
     assert np.array_equal(f.cpu().numpy(), [want, -want])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_fused_batch_window_overflow(cuda, precision):
+    """Two Morse gases that drift to their centres overflow the padded rows of
+    a fused graph window (odd and even lengths): the window is done again from
+    its start, with the bits of unfused windows whose rows overflow as well,
+    and of a single system."""
+    from tdmd_claude_b200 import (Box, FastPipelineScheduler, MorseParams, ReplicaBatch,
+                                  make_config)
+    rng = np.random.default_rng(3)
+    L, n = 30.0, 300
+    x = rng.uniform(0, L, size=(n, 3))
+    v, types, masses = 15.0 - x, np.ones(n, np.int32), np.array([1.0, 63.546])
+    boxes, p = [Box.make((0,) * 3, (L,) * 3)] * 2, MorseParams.make(0.01, 1.0, 3.0, 5.0)
+    for windows in ((200,), (99, 200)):
+        out = []
+        for graphs in (True, False):
+            cfg = make_config(r_skin=1.0, rebuild_every=5, dt=0.002, precision=precision,
+                              lanes_per_atom=8, use_graphs=graphs)
+            b = ReplicaBatch(boxes, [n, n], p, cfg)
+            b.upload(np.concatenate([x, x]), np.concatenate([v, 0.9 * v]),
+                     np.concatenate([types] * 2), masses)
+            s = FastPipelineScheduler(boxes[0], n, p, cfg)
+            s.upload(x, v, None, types, None, masses)
+            for t in windows:
+                b.run_until(t)
+                s.run_until(t)
+            assert b.stats().nlist_retries >= 1 and s.stats().nlist_retries >= 1
+            st = s.download()
+            out.append((b.download(), (st.positions, st.velocities, st.forces)))
+        (gb, gs), (ub, us) = out
+        for i in range(3):
+            assert np.array_equal(gb[i], ub[i]) and np.array_equal(gs[i], us[i])
+        for i in range(2):
+            assert np.array_equal(gb[i][:n], gs[i])
