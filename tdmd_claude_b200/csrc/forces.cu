@@ -283,6 +283,8 @@ void EamDevTables::upload(const tdmd_eam& e, cudaStream_t stream) {
                       static_cast<float>(1.0 / e.dr), static_cast<float>(e.cutoff * e.cutoff),
                       e.drho, static_cast<float>(e.dr - static_cast<double>(dr32)), tbits};
   d32.top = static_cast<unsigned>(std::min(e.nr - 2, (1 << 22) - 1));
+  d32.end = static_cast<float>(e.nr - 2);
+  if (static_cast<double>(d32.end) > e.nr - 2) d32.end = std::nextafterf(d32.end, 0.f);
 }
 
 // --------------------------------------------------------------------------

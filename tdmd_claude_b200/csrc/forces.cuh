@@ -219,11 +219,19 @@ __device__ __forceinline__ double root_d(double x) {
 
 // x / r: FP64 corrects the product with 1/r by its exact remainder (the
 // division's rounding; an infinite quotient has no remainder and stays, as the
-// division leaves it); FP32 multiplies by rsqrt.
+// division leaves it -- a predicate on the correction, which costs nothing
+// measurable, where selecting between the two took 0.5 % of the FP64 passes);
+// FP32 multiplies by rsqrt.
 __device__ __forceinline__ double div_r(double x, double r, double rinv) {
-  const double q = x * rinv;
-  const double c = fma(fma(-q, r, x), rinv, q);
-  return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : c;
+  double q = x * rinv;
+  const double rem = fma(-q, r, x);
+  asm("{\n .reg .pred finite;\n .reg .b32 lo, hi;\n"
+      " mov.b64 {lo, hi}, %0;\n and.b32 hi, hi, 0x7ff00000;\n"
+      " setp.ne.u32 finite, hi, 0x7ff00000;\n"
+      " @finite fma.rn.f64 %0, %1, %2, %0;\n}"
+      : "+d"(q)
+      : "d"(rem), "d"(rinv));
+  return q;
 }
 __device__ __forceinline__ float div_r(float x, float /*r*/, float rinv) { return x * rinv; }
 
@@ -776,9 +784,10 @@ struct EamDev {
   const double4* d4 = nullptr;
   const double2* d2 = nullptr;
   const double* da = nullptr;
-  // FP32 path: the last interval that spline_interval finds without a
-  // conversion, min(nr - 2, 2^22 - 1)
+  // FP32 path: the last interval that spline_interval reads from the bits,
+  // min(nr - 2, 2^22 - 1), and the table's last one as a float (not above it)
   unsigned top = 0;
+  float end = 0.f;
 };
 
 __device__ __forceinline__ int phi_slot(int ti, int tj, int nt) {
@@ -823,18 +832,19 @@ __device__ __forceinline__ int spline_idx_mul(double r, double dr, double inv_dr
 
 // Interval of r in FP32 and the same number as a float, as spline_idx_mul has
 // it in FP64: no conversions, which run at a quarter of the rate of the
-// additions that replace them.  From 2^22 on the sum with 1.5 * 2^23 is no
-// longer spaced by one, and beyond the table the last interval goes on: both
-// lie past e.top and take the conversion (r / dr is a whole float there, or the
-// interval is below 2^24: fi is exact).
+// additions that replace them.  From 2^22 on the sum with 1.5 * 2^23 is spaced
+// by two and more: its difference from 1.5 * 2^23 is still a whole number
+// within that spacing of r / dr - 1/2 (the offset goes with it, over smooth
+// neighboring cubics), but no longer the difference of the bits, so that these
+// intervals, and the last one beyond the table, take the conversion.
 __device__ __forceinline__ int spline_interval(float r, const EamDev<float>& e, float& fi) {
   constexpr float kRound = 12582912.f;  // 1.5 * 2^23
   const float z = __fadd_rn(fmaf(r, e.inv_dr, -0.5f), kRound);
   int idx = __float_as_int(z) - 0x4B400000;
   fi = __fsub_rn(z, kRound);
   if (static_cast<unsigned>(idx) > e.top) {
-    idx = min(static_cast<int>(r * e.inv_dr), e.nr - 2);
-    fi = static_cast<float>(idx);
+    fi = fminf(fi, e.end);
+    idx = static_cast<int>(fi);
   }
   return idx;
 }
