@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(kThreads) k_morse_atom_pe(Geo g, NbrView nl, i
 
 // Per-atom EAM energy F_ti(rho_i) + 1/2 sum_j phi(r_ij), with the force
 // pass's spline rows and offsets; only on energy-log windows.
-template <class Geo, int LPA, int U, bool VEC, bool MULTI>
+template <class Geo, int LPA, int U, bool VEC, bool MULTI, bool WIDE = false>
 __global__ void __launch_bounds__(kThreads) k_eam_atom_pe(Geo g, NbrView nl, int n,
                                                           EamDev<typename Geo::T> e,
                                                           const int* __restrict__ types,
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kThreads) k_eam_atom_pe(Geo g, NbrView nl, int
         if (pr.r2 < e.rc_sq) {
           T r, rinv, corr, sx;
           g.radius2(o, pr, r, rinv, corr);
-          const int idx = spline_at(r, corr, e, sx);
+          const int idx = spline_at<WIDE>(r, corr, e, sx);
           const int tj = MULTI ? __ldg(types + jj[u]) - 1 : 0;
           const auto cphi = ldv4<T>(e.rtab + static_cast<long long>(idx) * e.S +
                                     (MULTI ? phi_slot(ti, tj, e.ntypes) : 1));
@@ -998,24 +998,30 @@ void Batch::reduce_energies(double* out) {
   if (eam_) {
     // rho_i of the current positions, then F(rho_i) + 1/2 sum_j phi(r_ij)
     const int* types = eam_->ntypes > 1 ? types_.data() : nullptr;
+    auto atom_pe = [&](auto g, const auto& e) {
+      using Geo = decltype(g);
+      TDMD_MULTI_DISPATCH(types != nullptr, {
+        if (e.wide) {
+          launch(k_eam_atom_pe<Geo, 1, 2, false, M, true>, nblk, kThreads, 0, s, g, nl, n, e,
+                 types, rho_.data(), pe_atom_.data());
+        } else {
+          TDMD_VEC_DISPATCH(vec_rows(nl), TDMD_TUNE_DISPATCH(tn, {
+            launch(k_eam_atom_pe<Geo, L, U, V, M>, nblk, kThreads, 0, s, g, nl, n, e, types,
+                   rho_.data(), pe_atom_.data());
+          }));
+        }
+      });
+    };
     if (mixed_) {
       const GeoQB g{q_.data(), rep_.data(), scales_.data()};
       launch_eam_density<GeoQB, float>(g, nl, n, eam_->d32, types, fp32_.data(), rho_.data(),
                                        nullptr, g_.data(), false, nullptr, Tune{lpa_d_, nu_d_}, s);
-      TDMD_MULTI_DISPATCH(types != nullptr, TDMD_VEC_DISPATCH(vec_rows(nl), TDMD_TUNE_DISPATCH(
-          tn, {
-            launch(k_eam_atom_pe<GeoQB, L, U, V, M>, nblk, kThreads, 0, s, g, nl, n,
-                   eam_->d32, types, rho_.data(), pe_atom_.data());
-          })));
+      atom_pe(g, eam_->d32);
     } else {
       const GeoD4B g{pos4_.data(), rep_.data(), imgs_.data()};
       launch_eam_density<GeoD4B, double>(g, nl, n, eam_->d64, types, fp64_.data(), rho_.data(),
                                          nullptr, nullptr, false, nullptr, Tune{lpa_d_, nu_d_}, s);
-      TDMD_MULTI_DISPATCH(types != nullptr, TDMD_VEC_DISPATCH(vec_rows(nl), TDMD_TUNE_DISPATCH(
-          tn, {
-            launch(k_eam_atom_pe<GeoD4B, L, U, V, M>, nblk, kThreads, 0, s, g, nl, n,
-                   eam_->d64, types, rho_.data(), pe_atom_.data());
-          })));
+      atom_pe(g, eam_->d64);
     }
     TDMD_LAUNCH_CHECK();
     launches_ += 1;

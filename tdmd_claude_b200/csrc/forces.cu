@@ -282,9 +282,8 @@ void EamDevTables::upload(const tdmd_eam& e, cudaStream_t stream) {
   d32 = EamDev<float>{dtab32.data(), rtab32.data(), ftab.data(), nt, S, e.nr, e.nrho, dr32,
                       static_cast<float>(1.0 / e.dr), static_cast<float>(e.cutoff * e.cutoff),
                       e.drho, static_cast<float>(e.dr - static_cast<double>(dr32)), tbits};
-  d32.top = static_cast<unsigned>(std::min(e.nr - 2, (1 << 22) - 1));
-  d32.end = static_cast<float>(e.nr - 2);
-  if (static_cast<double>(d32.end) > e.nr - 2) d32.end = std::nextafterf(d32.end, 0.f);
+  d32.wide = e.nr > (1 << 22);
+  d64.wide = e.cutoff / e.dr >= 2147483648.0;
 }
 
 // --------------------------------------------------------------------------

@@ -784,10 +784,7 @@ struct EamDev {
   const double4* d4 = nullptr;
   const double2* d2 = nullptr;
   const double* da = nullptr;
-  // FP32 path: the last interval that spline_interval reads from the bits,
-  // min(nr - 2, 2^22 - 1), and the table's last one as a float (not above it)
-  unsigned top = 0;
-  float end = 0.f;
+  int wide = 0;  // read by the launches: the table takes the WIDE kernels (spline_at)
 };
 
 __device__ __forceinline__ int phi_slot(int ti, int tj, int nt) {
@@ -814,17 +811,15 @@ __device__ __forceinline__ int spline_idx(double r, double dr, int n, double& dx
 // Where q is within a rounding of a knot the neighboring interval may be
 // taken (every other exact knot goes to the one below): only for splines whose
 // value and derivative are continuous, as build_spline's are, so that the
-// result changes by a rounding only.  From 2^32 on (a cutoff far beyond the
-// table) the sum leaves the low word, which its high word shows.
+// result changes by a rounding only.  0 <= q < 2^31.
 __device__ __forceinline__ int spline_idx_mul(double r, double dr, double inv_dr, int n,
                                               double& dx) {
   constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52
   const double z = fma(r, inv_dr, -0.5) + kRound;
   int idx = __double2loint(z);
   dx = fma(-(z - kRound), dr, r);
-  if (static_cast<unsigned>(idx) > static_cast<unsigned>(n - 2) ||
-      __double2hiint(z) != 0x43380000) {
-    idx = n - 2;
+  if (static_cast<unsigned>(idx) > static_cast<unsigned>(n - 2)) {
+    idx = idx < 0 ? 0 : n - 2;
     dx = r - static_cast<double>(idx) * dr;
   }
   return idx;
@@ -832,19 +827,15 @@ __device__ __forceinline__ int spline_idx_mul(double r, double dr, double inv_dr
 
 // Interval of r in FP32 and the same number as a float, as spline_idx_mul has
 // it in FP64: no conversions, which run at a quarter of the rate of the
-// additions that replace them.  From 2^22 on the sum with 1.5 * 2^23 is spaced
-// by two and more: its difference from 1.5 * 2^23 is still a whole number
-// within that spacing of r / dr - 1/2 (the offset goes with it, over smooth
-// neighboring cubics), but no longer the difference of the bits, so that these
-// intervals, and the last one beyond the table, take the conversion.
+// additions that replace them.  0 <= r / dr < 2^22, and beyond the table.
 __device__ __forceinline__ int spline_interval(float r, const EamDev<float>& e, float& fi) {
   constexpr float kRound = 12582912.f;  // 1.5 * 2^23
   const float z = __fadd_rn(fmaf(r, e.inv_dr, -0.5f), kRound);
   int idx = __float_as_int(z) - 0x4B400000;
   fi = __fsub_rn(z, kRound);
-  if (static_cast<unsigned>(idx) > e.top) {
-    fi = fminf(fi, e.end);
-    idx = static_cast<int>(fi);
+  if (static_cast<unsigned>(idx) > static_cast<unsigned>(e.nr - 2)) {
+    idx = idx < 0 ? 0 : e.nr - 2;
+    fi = static_cast<float>(idx);
   }
   return idx;
 }
@@ -857,11 +848,28 @@ __device__ __forceinline__ int spline_interval(float r, const EamDev<float>& e, 
 // distance to spline row, and with the intervals above: mixed EAM 131k 3.87 ->
 // 3.82 ms per 50 steps, 1.05 M atoms 11.89 -> 11.73 ms per 20; ternary 55k NVT
 // and 2 767 atoms within their spread.
+//
+// WIDE: tables beyond the range of these intervals -- 2^22 knots and more in
+// FP32, a cutoff 2^31 spacings and more away in FP64 -- find them by division
+// and conversion, the offset in FP64.  Kernels of their own (EamDev::wide, by the
+// launch): the same cases on a rare branch here cost every mixed pass
+// 0.3-0.5 % and the multi-type force pass 1.6 %, and moved what the autotuner
+// picks for 4 M ternary atoms (24.5 -> 26.0 ms a window).
+template <bool WIDE>
 __device__ __forceinline__ int spline_at(double r, double /*corr*/, const EamDev<double>& e,
                                          double& sx) {
+  if constexpr (WIDE) return spline_idx(r, e.dr, e.nr, sx);
   return spline_idx_mul(r, e.dr, e.inv_dr, e.nr, sx);
 }
+template <bool WIDE>
 __device__ __forceinline__ int spline_at(float r, float corr, const EamDev<float>& e, float& sx) {
+  if constexpr (WIDE) {
+    const int idx = min(static_cast<int>(r * e.inv_dr), e.nr - 2);
+    sx = static_cast<float>(fma(-static_cast<double>(idx),
+                                static_cast<double>(e.dr) + static_cast<double>(e.dr_lo),
+                                static_cast<double>(r) + static_cast<double>(corr)));
+    return idx;
+  }
   float fi;
   const int idx = spline_interval(r, e, fi);
   sx = __fadd_rn(fmaf(-fi, e.dr, r), fmaf(-fi, e.dr_lo, corr));
@@ -869,12 +877,13 @@ __device__ __forceinline__ int spline_at(float r, float corr, const EamDev<float
 }
 
 // Interval and offset from r alone (density pass).
-template <class T>
+template <bool WIDE, class T>
 __device__ __forceinline__ int spline_fast(double r, const EamDev<T>& e, double& sx) {
-  return spline_idx_mul(r, e.dr, e.inv_dr, e.nr, sx);
+  return spline_at<WIDE>(r, 0.0, e, sx);
 }
-template <class T>
+template <bool WIDE, class T>
 __device__ __forceinline__ int spline_fast(float r, const EamDev<T>& e, float& sx) {
+  if constexpr (WIDE) return spline_at<true>(r, 0.f, e, sx);
   float fi;
   const int idx = spline_interval(r, e, fi);
   sx = fmaf(-fi, e.dr_lo, fmaf(-fi, e.dr, r));
@@ -949,7 +958,7 @@ __device__ __forceinline__ void embed_eval(const double4* ftab, int nrho, double
 // and, with EV, the embedding energy F(rho_i) into the block partials.
 // types == nullptr means a single-type alloy.  gout (GeoQ only, nullable)
 // receives the force pass's gather records {qx, qy, qz, bits(F'(rho))}.
-template <class Geo, int LPA, int U, bool EV, bool VEC, bool MULTI, class FP>
+template <class Geo, int LPA, int U, bool EV, bool VEC, bool MULTI, class FP, bool WIDE = false>
 __global__ void __launch_bounds__(256) k_eam_density(Geo g, NbrView nl, int n,
                                                      EamDev<typename Geo::T> e,
                                                      const int* __restrict__ types,
@@ -991,7 +1000,7 @@ __global__ void __launch_bounds__(256) k_eam_density(Geo g, NbrView nl, int n,
           // (the force pass's radius dominates), so it is not worth the
           // FP64 work.
           T sx;
-          const int idx = spline_fast(g.radius_fast(pr[u]), e, sx);
+          const int idx = spline_fast<WIDE>(g.radius_fast(pr[u]), e, sx);
           // fixed-point position records carry the atom's 1-based type in
           // their fourth word (the density pass always reads those)
           int tj = 0;
@@ -1045,7 +1054,7 @@ __global__ void __launch_bounds__(256) k_eam_density(Geo g, NbrView nl, int n,
 // instead of the fp array.  KD (FPG, float forces): then the next step's
 // kick + drift of the same atom.
 template <class Geo, int LPA, int U, int EV, bool FPG, bool VEC, bool MULTI, class FP, class F,
-          bool KD = false>
+          bool KD = false, bool WIDE = false>
 __global__ void __launch_bounds__(256) k_eam_force(Geo g, NbrView nl, int n,
                                                    EamDev<typename Geo::T> e,
                                                    const int* __restrict__ types,
@@ -1092,7 +1101,7 @@ __global__ void __launch_bounds__(256) k_eam_force(Geo g, NbrView nl, int n,
         if (pr[u].r2 < e.rc_sq) {
           T r, rinv, corr, sx;
           g.radius2(o, pr[u], r, rinv, corr);
-          const int idx = spline_at(r, corr, e, sx);
+          const int idx = spline_at<WIDE>(r, corr, e, sx);
           const int j = jj[u];
           int tj = 0;
           if constexpr (MULTI && FPG && Geo::kRecords)

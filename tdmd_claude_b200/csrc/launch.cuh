@@ -130,6 +130,20 @@ void launch_eam_density(const Geo& g, const NbrView& nl, int n,
                         Tune tn, cudaStream_t s, double* e_out = nullptr,
                         double4* gout64 = nullptr) {
   const int nblk = force_blocks(n, tn.lpa);
+  // Tables beyond the fast intervals: one shape, one lane an atom, on the
+  // grid (and with the partial records) of the shape that was asked for.
+  if (e.wide) {
+    TDMD_MULTI_DISPATCH(types != nullptr, {
+      if (ev)
+        launch(k_eam_density<Geo, 1, 2, true, false, M, FP, true>, nblk, kForceThreads, 0, s, g, nl,
+               n, e, types, fp, rho_out, fpd_out, gout, partials, e_out, gout64);
+      else
+        launch(k_eam_density<Geo, 1, 2, false, false, M, FP, true>, nblk, kForceThreads, 0, s, g,
+               nl, n, e, types, fp, rho_out, fpd_out, gout, nullptr, e_out, gout64);
+    });
+    TDMD_LAUNCH_CHECK();
+    return;
+  }
   TDMD_MULTI_DISPATCH(types != nullptr, TDMD_VEC_DISPATCH(vec_rows(nl), TDMD_TUNE_DISPATCH(tn, {
     if (ev)
       launch(k_eam_density<Geo, L, U, true, V, M, FP>, nblk, kForceThreads, 0, s, g, nl, n, e,
@@ -153,6 +167,27 @@ void launch_eam_force(const Geo& g, const NbrView& nl, int n, const EamDev<typen
                       Tune tn, cudaStream_t s, const KickDrift* kd = nullptr,
                       double* pe_atom = nullptr) {
   const int nblk = force_blocks(n, tn.lpa);
+  if (e.wide) {  // as in the density pass
+    const ForceOut<F> out{forces};
+    TDMD_MULTI_DISPATCH(types != nullptr, {
+      if (ev && !partials && pe_atom)
+        launch(k_eam_force<Geo, 1, 2, 2, FPG, false, M, FP, F, false, true>, nblk, kForceThreads, 0,
+               s, g, nl, n, e, types, fp, out, nullptr, KickDrift{}, pe_atom);
+      else if (ev)
+        launch(k_eam_force<Geo, 1, 2, 1, FPG, false, M, FP, F, false, true>, nblk, kForceThreads, 0,
+               s, g, nl, n, e, types, fp, out, partials, KickDrift{}, pe_atom);
+      else if (!kd)
+        launch(k_eam_force<Geo, 1, 2, 0, FPG, false, M, FP, F, false, true>, nblk, kForceThreads, 0,
+               s, g, nl, n, e, types, fp, out, nullptr, KickDrift{}, nullptr);
+      else if constexpr (FPG)
+        launch(k_eam_force<Geo, 1, 2, 0, FPG, false, M, FP, F, true, true>, nblk, kForceThreads, 0,
+               s, g, nl, n, e, types, fp, out, nullptr, *kd, nullptr);
+      else
+        TDMD_REQUIRE(false, "fused kick-drift needs a gather-record force pass");
+    });
+    TDMD_LAUNCH_CHECK();
+    return;
+  }
   TDMD_MULTI_DISPATCH(types != nullptr, TDMD_VEC_DISPATCH(vec_rows(nl), TDMD_TUNE_DISPATCH(tn, {
     if (ev && !partials && pe_atom)  // per-atom energies only
       launch(k_eam_force<Geo, L, U, 2, FPG, V, M, FP, F>, nblk, kForceThreads, 0, s, g, nl, n, e,

@@ -424,21 +424,61 @@ def _pair_eam(torch, eam, r, precision):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-def test_eam_table_of_five_million_knots(cuda, precision):
-    """Distances on both sides of 2^22 = 4.19 M knots, where an FP32 sum with
-    1.5 * 2^23 stops being spaced by one: density and force of smooth
+def test_eam_table_of_ten_million_knots(cuda, precision):
+    """Distances on both sides of 2^22 knots, where an FP32 sum with 1.5 * 2^23
+    stops being spaced by one, and of 2^23, past FP32 intervals: density and force of smooth
     functions (FP32 distance, product and sum roundings: 1e-6 and 3e-6)."""
     from tdmd_claude_b200 import EamAlloy
-    nr, dr = 5_000_001, 1e-6
+    nr, dr = 10_000_001, 5e-7
     x = np.arange(nr) * dr
     F = -0.5 * np.arange(100) * 0.1  # F' = -1/2
     eam = EamAlloy.from_tables(1, 100, 0.1, nr, dr, 5.0, F[None], np.exp(-x)[None],
                                (x * np.exp(-2 * x))[None])
-    rs = [2.5, (2 ** 22 - 3) * dr, (2 ** 22 + 3.5) * dr, 4.5, 4.9]
+    rs = [1.5, (2 ** 22 - 3) * dr, (2 ** 22 + 3.5) * dr, 2.9, (2 ** 23 - 3) * dr,
+          (2 ** 23 + 3.5) * dr, 4.5, 4.9]
     for r, (rho, fx) in zip(rs, _pair_eam(cuda, eam, rs, precision)):
         assert np.abs(rho / np.exp(-r) - 1).max() <= 1e-6
         want = -2 * np.exp(-2 * r) + np.exp(-r)  # phi' + 2 F' rho', on atom 0 along +x
         assert abs(fx - want) <= 3e-6 * np.exp(-r)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("ntypes", [1, 2])
+def test_wide_table_windows(cuda, precision, ntypes):
+    """Windows, energies and replicas with a table of 2^22 + 2 knots equal
+    those with one of 2000 knots of the same functions, to the coarse table's
+    interpolation and twice the mixed bound: 3e-5 of the largest force (1e-5
+    from the batch, which sums in another order)."""
+    from tdmd_claude_b200 import Box, EamAlloy, FastPipelineScheduler, ReplicaBatch, make_config
+    from tdmd_claude_b200 import workloads as W
+    rng = np.random.default_rng(2)
+    x = W.fcc_lattice(4, 4, 4, 3.615)
+    x = (x + rng.normal(0, 0.05, x.shape)) % (4 * 3.615)
+    n, box = len(x), Box.make((0,) * 3, (4 * 3.615,) * 3)
+    types = rng.integers(1, ntypes + 1, n).astype(np.int32)
+    masses = np.array([1.0] + [63.546] * ntypes)
+    kw = {} if ntypes == 1 else dict(beta_f=(4.8, 5.2), A_phi=(0.55, 0.65), E_F=(1.1, 1.3))
+    out = []
+    for nr in (2000, 2 ** 22 + 2):
+        t = W.analytic_eam(nr=nr, **kw)
+        eam = EamAlloy.from_tables(t.ntypes, t.nrho, t.drho, t.nr, t.dr, t.cutoff, t.F, t.rho,
+                                   t.rphi)
+        cfg = make_config(r_skin=0.3, precision=precision, energy_every=4, lanes_per_atom=8)
+        s = FastPipelineScheduler(box, n, eam, cfg)
+        s.upload(x, np.zeros((n, 3)), None, types, None, masses)
+        b = ReplicaBatch([box] * 2, [n, n], eam, cfg)
+        b.upload(np.concatenate([x, x]), np.zeros((2 * n, 3)), np.concatenate([types] * 2), masses)
+        for m in (s, b):
+            m.run_until(11)
+        pe, ke, w = s.energies()
+        bpe, bke = b.energies()
+        f = s.download().forces
+        assert np.abs(b.download()[2][:n] - f).max() <= 1e-5 * np.abs(f).max()
+        assert np.allclose(bpe, pe, rtol=1e-6) and np.allclose(bke, ke, rtol=1e-4)
+        out.append((f, pe, w))
+    (f0, e0, w0), (f1, e1, w1) = out
+    assert np.abs(f1 - f0).max() <= 3e-5 * np.abs(f0).max()
+    assert np.allclose(e1, e0, rtol=1e-6) and np.abs(w1 - w0).max() <= 1e-4 * np.abs(w0).max()
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
