@@ -771,8 +771,9 @@ void Scheduler::grow_capacity(int max_count) {
   want = (want + 7) / 8 * 8;
   TDMD_REQUIRE(want * std::max(n_, 1) < (1ll << 40), "neighbor list too large");
   if (want > cap_) {
+    cap_ = 0;  // no rows, should the allocation fail
+    nbr_.reserve(static_cast<size_t>(want) * static_cast<size_t>(std::max(n_, 1)));
     cap_ = static_cast<int>(want);
-    nbr_.reserve(static_cast<size_t>(cap_) * static_cast<size_t>(std::max(n_, 1)));
     clear_graphs();
   }
 }

@@ -219,3 +219,42 @@ for precision, refused in (("fp64", 3), ("mixed", 4), ("mixed", 5)):
         for x, y in zip(a, b):
             assert np.array_equal(x, y)
 """)
+
+
+def test_overflow_without_room_for_longer_rows(child):
+    """Rows that overflow in a window and cannot grow: the error is reported,
+    the state is the window's start, and the next window makes its rows anew
+    and reaches the state of an undisturbed run."""
+    child("""
+rng = np.random.default_rng(3)
+L, n = 30.0, 300
+x = rng.uniform(0, L, (n, 3))
+v, types, masses = 15.0 - x, np.ones(n, np.int32), np.array([1.0, 63.546])
+box = Box.make((0,) * 3, (L,) * 3)
+def make(batch):
+    cfg = make_config(r_skin=1.0, rebuild_every=5, dt=0.002, lanes_per_atom=8)
+    p = MorseParams.make(0.01, 1.0, 3.0, 5.0)
+    m = ReplicaBatch([box], [n], p, cfg) if batch else FastPipelineScheduler(box, n, p, cfg)
+    m.upload(x, v, types, masses) if batch else m.upload(x, v, None, types, None, masses)
+    m.run_until(5)
+    return m
+def state(m, batch):
+    d = m.download()
+    return [np.array(a) for a in (d[:2] if batch else (d.positions, d.velocities))]
+for batch in (False, True):
+    m, good = make(batch), make(batch)
+    assert good.stats().nlist_retries == 0
+    start = state(good, batch)
+    fail(b"cudaMalloc", 1, OOM)
+    try:
+        m.run_until(200)
+        raise SystemExit("no error")
+    except TdmdError as e:
+        assert "OUT_OF_MEMORY" in str(e), e
+    for a, b in zip(state(m, batch), start):
+        assert np.array_equal(a, b)
+    m.run_until(200), good.run_until(200)
+    assert good.stats().nlist_retries >= 1
+    d = state(m, batch)[0] - state(good, batch)[0]  # (the lists' steps differ)
+    assert np.abs(d - np.round(d / L) * L).max() <= 1e-8
+""")
