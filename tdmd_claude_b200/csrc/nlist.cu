@@ -996,7 +996,7 @@ int32_t tdmd_nlist_destroy(tdmd_nlist* nl) {
 // A handle's first build sweeps the candidates twice (count, device scan,
 // fill), like the reference.  Later builds know how long the longest row was:
 // one sweep fills rows padded to a quarter above that, and a copy packs them
-// (118 661 atoms, 53 neighbors: count pass 75 us against 10 us for the copy).
+// (118 661 atoms, 53 neighbors: count pass 75 us against 10 to 16 us for the copy).
 // A row that does not fit costs the second sweep again, from its exact
 // counts.  The padded rows are a convenience: they are bounded at 2 GiB and at
 // four times the last list plus 32 entries an atom (a crystal's take 1.7 times,

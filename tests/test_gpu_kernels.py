@@ -292,7 +292,8 @@ def test_device_eam_graphs_keep_their_scratch(cuda, precision):
             self.types = cuda.ones(self.n, dtype=cuda.int32, device="cuda")
             self.nl = DeviceNeighborList()
             self.nl.build(self.x, self.n, self.box, t.cutoff, 0.3)
-            self.e, self.w = (cuda.zeros(k, dtype=cuda.float64, device="cuda") for k in (1, 6))
+            self.e, self.w = (cuda.zeros(k, dtype=cuda.float64, device="cuda")
+                              for k in (1, 6))
             self.f = cuda.zeros((self.n, 3), device="cuda",
                                 dtype=cuda.float64 if precision == "fp64" else cuda.float32)
             cuda.cuda.synchronize()
@@ -342,8 +343,9 @@ def test_device_eam_graphs_keep_their_scratch(cuda, precision):
 @pytest.mark.parametrize("ntypes", [1, 3])
 def test_eam_fit_pairs_on_knots(cuda, oracle, a, dr, ntypes):
     """Ideal simple-cubic snapshots (with vacancies, so that the densities
-    differ) whose shells sit on spline knots, with coefficients that jump there: loss and gradient belong to the interval
-    int(r / dr), as in the oracle (the bounds of the other FP64 fits)."""
+    differ) whose shells sit on spline knots, with coefficients that jump
+    there: loss and gradient belong to the interval int(r / dr), as in the
+    oracle (the bounds of the other FP64 fits)."""
     from tdmd_claude_b200 import Box, EamAlloy
     from tdmd_claude_b200 import workloads as W
     from tdmd_claude_b200.fitting import ForceMatch, eam_coeff_tensors, eam_table_meta
